@@ -246,12 +246,8 @@ int ct_knn_residual(ct_tree* T, const int64_t* q_ids, int64_t nq, int32_t k, int
     if (stats) memset(stats, 0, sizeof(*stats));
     switch (form) {
         case CT_FORM_DENSE: {
-            int dev = 0;
-            CT_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
-            int smem_optin = 0;
-            CT_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "smem attr");
-            int qt = ct::brute_pick_qt(T->m, T->d, k, (size_t)smem_optin);
-            if (qt == 0) return fail(CT_ERR_UNSUPPORTED, "ct_knn_residual: m=%d, k=%d exceed shared memory", T->m, k);
+            if (!ct::brute_fits(T->m, T->d, k))
+                return fail(CT_ERR_UNSUPPORTED, "ct_knn_residual: m=%d, k=%d exceed shared memory", T->m, k);
             ct::BruteParams P;
             P.vperm = T->vperm; P.xs = T->xs; P.norms = T->norms; P.p = T->p;
             P.qids = (const long long*)q_ids; P.n = T->n; P.nq = nq; P.m = T->m; P.d = T->d; P.k = k;
@@ -263,7 +259,7 @@ int ct_knn_residual(ct_tree* T, const int64_t* q_ids, int64_t nq, int32_t k, int
                 CT_CUDA(cudaEventCreate(&e1), "event");
                 CT_CUDA(cudaEventRecord(e0, st), "event record");
             }
-            CT_CUDA(ct::launch_brute_knn(P, qt, st), "dense kNN launch");
+            CT_CUDA(ct::launch_brute_knn(P, true, st), "dense kNN launch");
             if (g_timing) {
                 float ms = 0.f;
                 CT_CUDA(cudaEventRecord(e1, st), "event record");

@@ -20,9 +20,13 @@
 // no memset and the launch sequence can be replayed as a CUDA graph:
 // [copy descriptors from pinned host memory, persistent kernel].
 //
-// The autotuner (ct_batch_autotune) times the candidate launch shapes —
-// queries per CTA tile (QT = 64 / 32 / 16), CTAs per SM, and the candidate split
-// target (work items per SM slot) — on the batch itself and keeps the fastest.
+// Each problem takes the tile height of its own query count (16 rows up to 16 queries, 32 above),
+// so small and large query sets of one launch are both free of padding; a launch runs two blocks
+// per SM unless a problem's rows are too wide (dense::Cfg).
+//
+// The autotuner (ct_batch_autotune) times the candidate launch shapes — queries per CTA tile
+// (32 / 16), CTAs per SM, and the candidate split target (work items per SM slot) — on the batch
+// itself and keeps the fastest.
 #include <cuda_runtime.h>
 #include <limits.h>
 #include <stdio.h>
@@ -42,77 +46,32 @@ namespace ct {
 namespace batch {
 
 struct Problem {
-    dense::Tile base;     // q0 / cbeg / cend / out_* are set per item
-    long long tiles;      // query tiles of QT
-    long long chunk;      // candidates per chunk (multiple of dense::kCT)
+    dense::Tile base;     // q0 / cbeg / cend / part are set per item
+    long long tiles;      // query tiles of the problem's configuration
+    long long chunk;      // candidates per chunk (a multiple of the configuration's step)
     long long item_base;  // first work item of the problem
-    long long* part_idx;  // [nq][split][k] partial lists (split > 1)
-    float* part_dist;
+    dense::u64* part;     // [nq][split][k] partial lists of sorted keys (split > 1)
     int* tile_done;       // [tiles] chunk completion counters (split > 1)
     int split;            // candidate chunks per tile (1..kMaxSplit)
-    int pad_;
+    int cfg;              // tile configuration (dense::Cfg)
 };
 
 struct Header {
     long long total_items;
     int nprob;
-    int qt;
+    int pad_;
 };
 
 constexpr size_t kHeaderBytes = 64;
 
-// Merge a tile's `split` sorted partial lists per query into the final top-k.
-// One warp per query; lane l owns lists l, l+32, l+64 and l+96 and offers the
-// smallest of their heads to a warp-wide (dist, idx) minimum.
 constexpr int kMaxSplit = 128;
-__device__ void merge_partials(const Problem& B, long long tile, int QT) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k = B.base.k, S = B.split;
-    const float kInf = __int_as_float(0x7f800000);
-    for (int qi = warp; qi < QT; qi += dense::kThreads / 32) {
-        const long long g = tile * QT + qi;
-        if (g >= B.base.nq) continue;
-        int pos[4] = {0, 0, 0, 0};
-        float hd[4];
-        long long hi[4];
-        auto load = [&](int h) {
-            const int list = lane + 32 * h;
-            hd[h] = kInf;
-            hi[h] = LLONG_MAX;
-            if (list < S && pos[h] < k) {
-                const long long off = (g * S + list) * k + pos[h];
-                const long long i = __ldcg(B.part_idx + off);
-                if (i >= 0) { hi[h] = i; hd[h] = __ldcg(B.part_dist + off); }
-            }
-        };
-#pragma unroll
-        for (int h = 0; h < 4; ++h) load(h);
-        for (int j = 0; j < k; ++j) {
-            int bh = 0;
-#pragma unroll
-            for (int h = 1; h < 4; ++h)
-                if (nb_less(hd[h], hi[h], hd[bh], hi[bh])) bh = h;
-            float bd = hd[bh];
-            long long bi = hi[bh];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-                const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (nb_less(od, oi, bd, bi)) { bd = od; bi = oi; }
-            }
-            if (lane == 0) {
-                const bool pad = bi == LLONG_MAX;
-                B.base.out_idx[g * k + j] = pad ? -1LL : bi;
-                B.base.out_dist[g * k + j] = pad ? CT_FLT_MAX : bd;
-            }
-            if (bi != LLONG_MAX && hi[bh] == bi) { ++pos[bh]; load(bh); }
-        }
-    }
-}
 
-template <int QT, int MINB>
-__global__ void __launch_bounds__(dense::kThreads, MINB)
-    batch_kernel(const unsigned char* __restrict__ desc, unsigned long long* __restrict__ ctr) {
+// One launch serves problems of every tile height: each problem carries its own configuration.
+// NT = 256: the forms that run two blocks per SM; NT = 512: the forms for wide rows, when a
+// problem of the batch fits no other.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+    batch_kernel(const unsigned char* __restrict__ desc, unsigned long long* __restrict__ ctr, dense::u64 nz) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ dense::Tile sJ;
     __shared__ long long s_item;
@@ -137,28 +96,31 @@ __global__ void __launch_bounds__(dense::kThreads, MINB)
                 const long long tile = B.tiles - 1 - local / B.split;
                 const int chunk = (int)(local % B.split);
                 dense::Tile J = B.base;
-                J.q0 = tile * QT;
+                J.q0 = tile * dense::cfg_qt(B.cfg);
                 J.cbeg = (long long)chunk * B.chunk;
                 J.cend = J.cbeg + B.chunk < J.n ? J.cbeg + B.chunk : J.n;
-                if (B.split > 1) {
-                    J.out_idx = B.part_idx + (long long)chunk * J.k;
-                    J.out_dist = B.part_dist + (long long)chunk * J.k;
-                    J.out_stride = (long long)B.split * J.k;
-                } else {
-                    J.out_stride = J.k;
-                }
+                J.part = B.split > 1 ? B.part + (long long)chunk * J.k : nullptr;
+                J.part_stride = (long long)B.split * J.k;
                 sJ = J;
             }
         }
         __syncthreads();
         const long long it = s_item;
         if (it >= total) break;
-        dense::run_tile<QT>(sJ, smem_raw);
         const Problem& B = probs[s_prob];
+        const int cfg = B.cfg;
+        if constexpr (NT == 256) {
+            if (cfg == dense::kCfg32) dense::run_tile<dense::kCfg32>(sJ, nz);
+            else dense::run_tile<dense::kCfg16>(sJ, nz);
+        } else {
+            if (cfg == dense::kCfg32w) dense::run_tile<dense::kCfg32w>(sJ, nz);
+            else dense::run_tile<dense::kCfg16w>(sJ, nz);
+        }
         if (B.split > 1) {
             __threadfence();
             __syncthreads();
-            const long long tile = sJ.q0 / QT;
+            const int qt = dense::cfg_qt(cfg);
+            const long long tile = sJ.q0 / qt;
             if (threadIdx.x == 0) {
                 const int prev = atomicAdd(&B.tile_done[tile], 1);
                 s_last = prev == B.split - 1;
@@ -166,7 +128,9 @@ __global__ void __launch_bounds__(dense::kThreads, MINB)
             __syncthreads();
             if (s_last) {
                 __threadfence();
-                merge_partials(B, tile, QT);
+                const int nv = (int)(sJ.nq - sJ.q0 < qt ? sJ.nq - sJ.q0 : qt);
+                dense::merge_tile<NT>(B.part, B.split, sJ.k, sJ.q0, nv, (dense::u64*)smem_raw, sJ.out_idx,
+                                      sJ.out_dist, sJ.k);
                 if (threadIdx.x == 0) B.tile_done[tile] = 0;
             }
         }
@@ -183,17 +147,13 @@ __global__ void __launch_bounds__(dense::kThreads, MINB)
     }
 }
 
-typedef void (*KernelFn)(const unsigned char*, unsigned long long*);
+typedef void (*KernelFn)(const unsigned char*, unsigned long long*, dense::u64);
 
 struct Shape {
     int qt, cps;
 };
 
-KernelFn kernel_for(int qt, int cps) {
-    if (qt == 64) return batch_kernel<64, 1>;
-    if (qt == 32) return batch_kernel<32, 1>;
-    return cps >= 2 ? batch_kernel<16, 2> : batch_kernel<16, 1>;
-}
+KernelFn kernel_for(bool wide) { return wide ? batch_kernel<512> : batch_kernel<256>; }
 
 }  // namespace batch
 }  // namespace ct
@@ -232,7 +192,8 @@ struct ct_batch {
     // graph of [descriptor copy, kernel]
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t gexec = nullptr;
-    int g_qt = 0, g_cps = 0, g_grid = 0;
+    KernelFn g_fn = nullptr;
+    int g_grid = 0;
     size_t g_smem = 0, g_cap = 0;
     cudaEvent_t staged = nullptr;
     bool staged_pending = false;
@@ -283,21 +244,43 @@ int batch_init(ct_batch* B) {
 // static shared memory of the batch kernel (sJ and the item scalars)
 constexpr size_t kStaticSmem = sizeof(dense::Tile) + 64;
 
-size_t smem_for(const ct_batch* B, int qt) {
-    int m = B->res_m, d = B->res_d, k = B->res_k;
-    for (const BatchReq& r : B->reqs) {
-        m = std::max(m, r.tree->m);
-        d = std::max(d, r.tree->d);
-        k = std::max(k, r.k);
-    }
-    return dense::layout(qt, m, d, k).total;
+// A problem's configuration in a launch of the given kind: the 32-row form when it fits and the
+// height (0 = automatic) allows it, the 16-row form for up to 16 queries or when the other does
+// not fit.  False when neither fits.
+struct Config {
+    int cfg = 0;
+    dense::Ring ring{};
+    size_t smem = 0;
+};
+bool config_for(const ct_batch* B, int m, int d, int k, long long nq, int qt, bool wide, Config* c) {
+    const int tall = wide ? dense::kCfg32w : dense::kCfg32, low = wide ? dense::kCfg16w : dense::kCfg16;
+    const size_t limit = dense::cfg_limit(tall, B->smem_optin, B->smem_per_sm, kStaticSmem);
+    c->cfg = tall;
+    if (qt != 16 && (qt != 0 || nq > 16) && dense::pick_ring(tall, m, d, k, limit, &c->ring, &c->smem)) return true;
+    c->cfg = low;
+    return dense::pick_ring(low, m, d, k, limit, &c->ring, &c->smem);
 }
 
-bool shape_fits(const ct_batch* B, int qt, int cps) {
-    const size_t s = smem_for(B, qt);
-    if (s + kStaticSmem > B->smem_optin) return false;
-    if (cps >= 2 && (qt != 16 || 2 * (s + kStaticSmem + 1024) > B->smem_per_sm)) return false;
+bool all_fit(const ct_batch* B, bool wide) {
+    Config c;
+    if (!config_for(B, B->res_m, B->res_d, B->res_k, 1, 0, wide, &c)) return false;
+    for (const BatchReq& r : B->reqs)
+        if (!config_for(B, r.tree->m, r.tree->d, r.k, r.nq, 0, wide, &c)) return false;
     return true;
+}
+// Rows too wide for two blocks per SM take the whole batch to the 512-thread kernel.
+bool is_wide(const ct_batch* B) { return !all_fit(B, false); }
+
+// Shared memory of a launch: the largest of the batch's problems and of the reserved (m, d, k) in
+// either height.
+size_t smem_for(const ct_batch* B, int qt, bool wide) {
+    size_t most = 0;
+    Config c;
+    for (const BatchReq& r : B->reqs)
+        if (config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, wide, &c)) most = std::max(most, c.smem);
+    for (int nq = 16; nq <= 32; nq += 16)
+        if (config_for(B, B->res_m, B->res_d, B->res_k, nq, qt, wide, &c)) most = std::max(most, c.smem);
+    return most;
 }
 
 struct Plan {
@@ -306,19 +289,29 @@ struct Plan {
     size_t part_bytes = 0, done_ints = 0;
 };
 
+// The tallest tile of a plan (what ct_batch_get_shape reports for an automatic launch).
+int plan_qt(const Plan& P) {
+    int qt = 16;
+    for (const Problem& pr : P.probs) qt = std::max(qt, dense::cfg_qt(pr.cfg));
+    return qt;
+}
+
 // Order problems, choose each problem's candidate split and lay out its scratch.
-void make_plan(const ct_batch* B, int qt, int cps, int ips, Plan& P) {
+void make_plan(const ct_batch* B, int qt, int cps, int ips, bool wide, Plan& P) {
     const int nr = (int)B->reqs.size();
     std::vector<int> ord;
     std::vector<double> tile_work(nr, 0.0);
+    std::vector<Config> cfgs(nr);
     double total_work = 0.0;
     long long total_tiles = 0;
     for (int i = 0; i < nr; ++i) {
         const BatchReq& r = B->reqs[i];
         if (r.nq <= 0) continue;
-        const long long tiles = (r.nq + qt - 1) / qt;
+        config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, wide, &cfgs[i]);
+        const int height = dense::cfg_qt(cfgs[i].cfg);
+        const long long tiles = (r.nq + height - 1) / height;
         const double per_pair = (double)r.tree->m + 4.0 * r.tree->d + 16.0;
-        tile_work[i] = (double)r.tree->n * (r.predecessor ? 0.5 : 1.0) * qt * per_pair;
+        tile_work[i] = (double)r.tree->n * (r.predecessor ? 0.5 : 1.0) * height * per_pair;
         total_work += tile_work[i] * tiles;
         total_tiles += tiles;
         ord.push_back(i);
@@ -341,7 +334,10 @@ void make_plan(const ct_batch* B, int qt, int cps, int ips, Plan& P) {
         J.qv = r.qv; J.qcoords = r.qcoords; J.qp = r.qp; J.inv_ls = T->inv_ls;
         J.nq = r.nq;
         J.out_idx = (long long*)r.out_idx; J.out_dist = r.out_dist; J.out_stride = r.k;
-        pr.tiles = (r.nq + qt - 1) / qt;
+        pr.cfg = cfgs[i].cfg;
+        J.ring = cfgs[i].ring;
+        const int ct = dense::cfg_ct(pr.cfg), height = dense::cfg_qt(pr.cfg);
+        pr.tiles = (r.nq + height - 1) / height;
         // split so that the batch has about target_items items, in proportion to work
         int split = 1;
         if ((double)total_tiles < target_items && total_work > 0) {
@@ -349,8 +345,8 @@ void make_plan(const ct_batch* B, int qt, int cps, int ips, Plan& P) {
             split = (int)std::min((double)kMaxSplit, std::max(1.0, want));
         }
         long long chunk = (T->n + split - 1) / split;
-        chunk = ((chunk + dense::kCT - 1) / dense::kCT) * dense::kCT;
-        if (chunk < dense::kCT) chunk = dense::kCT;
+        chunk = ((chunk + ct - 1) / ct) * ct;
+        if (chunk < ct) chunk = ct;
         split = (int)((T->n + chunk - 1) / chunk);
         pr.split = split;
         pr.chunk = chunk;
@@ -358,10 +354,8 @@ void make_plan(const ct_batch* B, int qt, int cps, int ips, Plan& P) {
         item += pr.tiles * split;
         if (split > 1) {
             const size_t entries = (size_t)r.nq * split * r.k;
-            pr.part_idx = (long long*)(uintptr_t)part_off;  // offsets until the arena is known
+            pr.part = (dense::u64*)(uintptr_t)part_off;  // an offset until the arena is known
             part_off += (entries * 8 + 255) & ~size_t(255);
-            pr.part_dist = (float*)(uintptr_t)part_off;
-            part_off += (entries * 4 + 255) & ~size_t(255);
             pr.tile_done = (int*)(uintptr_t)(done_off * sizeof(int));
             done_off += (size_t)pr.tiles;
         }
@@ -418,17 +412,18 @@ int ensure_capacity(ct_batch* B, const Plan& P, cudaStream_t st) {
 
 int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_t st) {
     Plan P;
-    make_plan(B, qt, cps, ips, P);
+    const bool wide = is_wide(B);
+    if (wide) cps = 1;
+    make_plan(B, qt, cps, ips, wide, P);
     B->last_items = P.total_items;
     B->last_pairs = P.pairs;
-    B->last_qt = qt; B->last_cps = cps; B->last_ips = ips;
+    B->last_qt = qt ? qt : plan_qt(P); B->last_cps = cps; B->last_ips = ips;
     if (P.total_items == 0) return CT_OK;
     int rc = ensure_capacity(B, P, st);
     if (rc != CT_OK) return rc;
     for (Problem& pr : P.probs) {
         if (pr.split > 1) {
-            pr.part_idx = (long long*)(B->d_part + (uintptr_t)pr.part_idx);
-            pr.part_dist = (float*)(B->d_part + (uintptr_t)pr.part_dist);
+            pr.part = (dense::u64*)(B->d_part + (uintptr_t)pr.part);
             pr.tile_done = (int*)((unsigned char*)B->d_done + (uintptr_t)pr.tile_done);
         }
     }
@@ -442,13 +437,13 @@ int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_
     memset(&h, 0, sizeof(h));
     h.total_items = P.total_items;
     h.nprob = (int)P.probs.size();
-    h.qt = qt;
     memcpy(B->h_desc, &h, sizeof(h));
     memcpy(B->h_desc + kHeaderBytes, P.probs.data(), sizeof(Problem) * P.probs.size());
     const size_t copy_bytes = kHeaderBytes + sizeof(Problem) * P.probs.size();
 
-    const size_t smem = smem_for(B, qt);
-    KernelFn fn = kernel_for(qt, cps);
+    const size_t smem = smem_for(B, qt, wide);
+    const unsigned threads = wide ? 512 : 256;
+    KernelFn fn = kernel_for(wide);
     cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: shared-memory attribute");
     long long grid = (long long)B->num_sms * cps;
@@ -457,7 +452,7 @@ int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_
     B->last_grid = (int)grid;
 
     if (use_graph) {
-        if (!B->gexec || B->g_qt != qt || B->g_cps != cps || B->g_grid != (int)grid || B->g_smem != smem ||
+        if (!B->gexec || B->g_fn != fn || B->g_grid != (int)grid || B->g_smem != smem ||
             B->g_cap != B->desc_cap) {
             if (B->gexec) { cudaGraphExecDestroy(B->gexec); B->gexec = nullptr; }
             cudaGraph_t g = nullptr;
@@ -465,20 +460,20 @@ int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_
             if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: begin capture");
             // the whole descriptor buffer is copied: the graph is reusable for any batch that fits
             cudaMemcpyAsync(B->d_desc, B->h_desc, B->desc_cap, cudaMemcpyHostToDevice, B->cap_stream);
-            fn<<<(unsigned)grid, dense::kThreads, smem, B->cap_stream>>>(B->d_desc, B->d_ctr);
+            fn<<<(unsigned)grid, threads, smem, B->cap_stream>>>(B->d_desc, B->d_ctr, dense::kNegZero2);
             e = cudaStreamEndCapture(B->cap_stream, &g);
             if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: end capture");
             e = cudaGraphInstantiate(&B->gexec, g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) { B->gexec = nullptr; return B->cuda_err(e, "ct_batch: graph instantiate"); }
-            B->g_qt = qt; B->g_cps = cps; B->g_grid = (int)grid; B->g_smem = smem; B->g_cap = B->desc_cap;
+            B->g_fn = fn; B->g_grid = (int)grid; B->g_smem = smem; B->g_cap = B->desc_cap;
         }
         e = cudaGraphLaunch(B->gexec, st);
         if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: graph launch");
     } else {
         e = cudaMemcpyAsync(B->d_desc, B->h_desc, copy_bytes, cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: descriptor copy");
-        fn<<<(unsigned)grid, dense::kThreads, smem, st>>>(B->d_desc, B->d_ctr);
+        fn<<<(unsigned)grid, threads, smem, st>>>(B->d_desc, B->d_ctr, dense::kNegZero2);
         e = cudaGetLastError();
         if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: kernel launch");
     }
@@ -490,24 +485,8 @@ int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_
 
 void default_shape(const ct_batch* B, int& qt, int& cps, int& ips) {
     qt = B->cfg_qt;
-    cps = B->cfg_cps > 0 ? B->cfg_cps : 1;
+    cps = B->cfg_cps > 0 ? B->cfg_cps : 2;
     ips = B->cfg_ips > 0 ? B->cfg_ips : 4;
-    if (qt == 0) {
-        // the tile height whose padded work, weighted by the measured per-pair cost of
-        // the narrower tiles (more shared-memory traffic per multiply), is smallest
-        const int order[3] = {64, 32, 16};
-        const double cost[3] = {1.0, 1.6, 2.6};
-        double best = -1.0;
-        qt = 16;
-        for (int t = 0; t < 3; ++t) {
-            if (!shape_fits(B, order[t], 1)) continue;
-            double w = 0.0;
-            for (const BatchReq& r : B->reqs)
-                w += (double)((r.nq + order[t] - 1) / order[t]) * order[t] * (double)r.tree->n * cost[t];
-            if (best < 0.0 || w < best) { best = w; qt = order[t]; }
-        }
-    }
-    if (!shape_fits(B, qt, cps)) cps = 1;
 }
 
 }  // namespace
@@ -610,7 +589,7 @@ int ct_batch_run(ct_batch* B, int32_t use_graph, ct_stats* stats, void* stream) 
         if (r.tree->m % 16 != 0) return ct::batch_fail("ct_batch_run", "tree rank m must be a multiple of 16", CT_ERR_UNSUPPORTED);
     int qt, cps, ips;
     default_shape(B, qt, cps, ips);
-    if (!shape_fits(B, qt, cps))
+    if (is_wide(B) && !all_fit(B, true))
         return ct::batch_fail("ct_batch_run", "the batch's largest m, d, k exceed shared memory", CT_ERR_UNSUPPORTED);
     cudaStream_t st = (cudaStream_t)stream;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -645,7 +624,10 @@ int ct_batch_autotune(ct_batch* B, int32_t reps, void* stream, int32_t* qt_out, 
     if (!B) return ct::batch_fail("ct_batch_autotune", "batch is NULL", CT_ERR_ARG);
     cudaStream_t st = (cudaStream_t)stream;
     if (reps <= 0) reps = 1;
-    const Shape shapes[4] = {{64, 1}, {32, 1}, {16, 1}, {16, 2}};
+    const Shape shapes[4] = {{32, 2}, {32, 1}, {16, 2}, {16, 1}};
+    const bool wide = is_wide(B);
+    if (wide && !all_fit(B, true))
+        return ct::batch_fail("ct_batch_autotune", "no launch shape fits shared memory", CT_ERR_UNSUPPORTED);
     const int ipss[3] = {1, 4, 16};
     float best = 3.4e38f;
     int bq = 0, bc = 0, bi = 0;
@@ -654,13 +636,13 @@ int ct_batch_autotune(ct_batch* B, int32_t reps, void* stream, int32_t* qt_out, 
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     for (const Shape& s : shapes) {
-        if (!shape_fits(B, s.qt, s.cps)) continue;
+        if (wide && s.cps > 1) continue;
         std::vector<std::vector<int>> seen;  // split patterns already timed for this shape
         for (int ips : ipss) {
             Plan P;
-            make_plan(B, s.qt, s.cps, ips, P);
+            make_plan(B, s.qt, s.cps, ips, wide, P);
             std::vector<int> splits;
-            for (const Problem& pr : P.probs) splits.push_back(pr.split);
+            for (const Problem& pr : P.probs) { splits.push_back(pr.split); splits.push_back(pr.cfg); }
             if (std::find(seen.begin(), seen.end(), splits) != seen.end()) continue;  // same launch
             seen.push_back(splits);
             int rc = CT_OK;

@@ -378,7 +378,7 @@ int ct_tree::grow_tree(const ct_tree* base, cudaStream_t st) {
         bound = ct::make_bound_model(m, d, kernel_type, var, vmax, nmax);
     }
 
-    // node-order residue-major V for the dense searches of the build (freed at the end)
+    // node-order permuted V for the dense searches of the build (freed at the end)
     float* tvperm = nullptr;
     A((void**)&tvperm, sizeof(float) * N * m);
     if (e == cudaSuccess) {
@@ -402,9 +402,6 @@ int ct_tree::grow_tree(const ct_tree* base, cudaStream_t st) {
     A((void**)&lvl, 4 * gmax); A((void**)&deg, 4 * (gmax + 1)); A((void**)&cursor, 4 * (gmax + 1));
     A((void**)&indptr, 8 * (gmax + 1)); A((void**)&indices, 8 * gmax * 2 * kc); A((void**)&w, 4 * gmax * 2 * kc);
     A((void**)&sel, gmax); A((void**)&counters, 16);
-    int smem_optin = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e == cudaSuccess && n_tree > 0 && n_tree_base == 0) {
         set_root_kernel<<<1, 1, 0, st>>>(parents, levels);
         e = cudaGetLastError();
@@ -420,17 +417,13 @@ int ct_tree::grow_tree(const ct_tree* base, cudaStream_t st) {
         iota_kernel<<<gridn(g, 256), 256, 0, st>>>(s, g, gq);
         // traversal: nearest node of the tree built so far, nodes [0, s)
         BP.qids = gq; BP.nq = g; BP.k = 1; BP.cbeg = 0; BP.cend = s; BP.out_idx = t_idx; BP.out_dist = t_d;
-        int qt = ct::brute_pick_qt(m, d, 1, (size_t)smem_optin);
-        if (qt == 0) { e = cudaErrorInvalidValue; break; }
-        e = ct::launch_brute_knn(BP, qt, st);
+        e = ct::launch_brute_knn(BP, true, st);
         if (e != cudaSuccess) break;
         group_level_kernel<<<gridn(g, 256), 256, 0, st>>>(s, g, t_idx, t_d, levels, lvl);
         // conflict candidates: nearest group members (the point itself among them)
         const int kk = (int)std::min<long long>(kc, g);
         BP.k = kk; BP.cbeg = s; BP.cend = s + g; BP.out_idx = c_idx; BP.out_dist = c_d;
-        qt = ct::brute_pick_qt(m, d, kk, (size_t)smem_optin);
-        if (qt == 0) { e = cudaErrorInvalidValue; break; }
-        e = ct::launch_brute_knn(BP, qt, st);
+        e = ct::launch_brute_knn(BP, true, st);
         if (e != cudaSuccess) break;
         e = cudaMemsetAsync(deg, 0, 4 * (g + 1), st);
         if (e != cudaSuccess) break;

@@ -10,7 +10,7 @@ namespace ct {
 bool timing_enabled();
 
 struct BruteParams {
-    const float* vperm;   // n x m, residue-major columns (see ct_setup.cu)
+    const float* vperm;   // n x m, the dense tile's column order (see ct_setup.cu)
     const float* xs;      // n x d scaled coordinates
     const float* norms;   // n squared scaled norms
     const float* p;       // n residual variances
@@ -24,9 +24,11 @@ struct BruteParams {
     long long cbeg = 0, cend = 0;
 };
 
-size_t brute_smem_bytes(int qt, int m, int d, int k);
-int brute_pick_qt(int m, int d, int k, size_t smem_limit);
-cudaError_t launch_brute_knn(const BruteParams& P, int qt, cudaStream_t stream);
+// Whether some tile configuration holds (m, d, k) in the current device's shared memory.
+bool brute_fits(int m, int d, int k);
+// `scratch_ok`: the call may take stream-ordered scratch to split the candidates of a few query
+// tiles over the chip (not under stream capture, not for the allocation-free entry point).
+cudaError_t launch_brute_knn(const BruteParams& P, bool scratch_ok, cudaStream_t stream);
 
 // ct_setup.cu
 cudaError_t launch_metric_setup(const float* v, const float* p, const float* coords, long long n, int m, int d,

@@ -6,7 +6,7 @@
 // GPU through its own pool and forbids other allocators, or a latency-critical
 // loop that cannot afford the implicit device synchronisation of
 // cudaMalloc/cudaFree.  They pass inputs and outputs; everything the dense
-// kernel needs beyond them (the residue-major V copy, scaled coordinates, norms,
+// kernel needs beyond them (the permuted V copy, scaled coordinates, norms,
 // p copy, 1/lengthscale) lives in one file-scope __device__ array of fixed size,
 // reserved when the library is loaded and held by every GPU that loads it until
 // the process exits.
@@ -50,7 +50,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 }  // namespace
 
 // Scratch bytes a call needs: five pieces, each rounded up to a multiple of 256
-// bytes — V in residue-major order (4 n m), scaled coordinates (4 n d), squared norms
+// bytes — V in the dense tile's column order (4 n m), scaled coordinates (4 n d), squared norms
 // (4 n), p (4 n) and the inverse lengthscales (256).
 size_t ct_noalloc_bytes_needed(long long n, int m, int d) {
     return align256((size_t)n * m * 4) + align256((size_t)n * d * 4) + align256((size_t)n * 4) +
@@ -127,13 +127,7 @@ int ct_noalloc_dense_impl(const float* v, const float* p, const float* coords, l
     void* base = nullptr;
     int rc = noalloc_scratch(&base, err, errlen);
     if (rc != CT_OK) return rc;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int smem_optin = 0;
-    cudaError_t e = cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e != cudaSuccess) { snprintf(err, errlen, "device attribute: %s", cudaGetErrorString(e)); return CT_ERR_CUDA; }
-    const int qt = ct::brute_pick_qt(m, d, k, (size_t)smem_optin);
-    if (qt == 0) { snprintf(err, errlen, "m=%d, k=%d exceed shared memory", m, k); return CT_ERR_UNSUPPORTED; }
+    if (!ct::brute_fits(m, d, k)) { snprintf(err, errlen, "m=%d, k=%d exceed shared memory", m, k); return CT_ERR_UNSUPPORTED; }
     // carve the scratch: every byte is written below before it is read, so
     // nothing has to be cleared between calls
     unsigned char* b = (unsigned char*)base;
@@ -151,7 +145,7 @@ int ct_noalloc_dense_impl(const float* v, const float* p, const float* coords, l
         ils.v[i] = 1.0f / safe;  // ResidualMetric::new, src/metric.rs:93-101
     }
     write_inv_ls_kernel<<<1, 64, 0, st>>>(ils, d, inv_ls);
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = ct::launch_metric_setup(v, p, coords, n, m, d, inv_ls, vperm, xs, norms, pc, st);
     if (e == cudaSuccess) {
         ct::BruteParams P;
@@ -159,7 +153,7 @@ int ct_noalloc_dense_impl(const float* v, const float* p, const float* coords, l
         P.qids = q_ids; P.n = n; P.nq = nq; P.m = m; P.d = d; P.k = k;
         P.kernel_type = kernel_type == 1 ? 1 : 0; P.predecessor = predecessor ? 1 : 0; P.var = variance;
         P.out_idx = out_idx; P.out_dist = out_dist;
-        e = ct::launch_brute_knn(P, qt, st);
+        e = ct::launch_brute_knn(P, false, st);  // no scratch: one chunk per query tile
     }
     if (e != cudaSuccess) { snprintf(err, errlen, "%s", cudaGetErrorString(e)); return CT_ERR_CUDA; }
     return CT_OK;

@@ -3,11 +3,13 @@
 // build_pcct2_residual_tree, src/lib.rs:1404-1439).
 //
 // HBM layout written here:
-//   vperm [n x m] f32  residue-major V: column l*(m/16)+c holds V[:, 16c+l]
+//   vperm [n x m] f32  V in the dense tile's column order (dense::perm_col): lanes l and
+//                      l + 8 of the reference's sixteen accumulators side by side
 //   xs    [n x d] f32  coords * (1/lengthscale), rounded exactly as the reference
 //   norms [n]     f32  sum of xs^2, left to right
 //   p     [n]     f32  residual variances (copy)
 #include "ct_common.cuh"
+#include "ct_dense.cuh"
 #include "ct_internal.h"
 
 namespace ct {
@@ -28,16 +30,17 @@ __global__ void setup_rows_kernel(const float* __restrict__ coords, const float*
     pcopy[r] = p[r];
 }
 
-// vperm[r, l*m16 + c] = v[r, 16c + l]
+// vperm[r, perm_col(col)] = v[r, col], one thread per output column
 __global__ void permute_v_kernel(const float* __restrict__ v, long long n, int m, float* __restrict__ vperm) {
-    const int m16 = m / 16;
-    long long total = n * (long long)m;
+    const int rw = m >> 3;
+    const long long total = n * (long long)m;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
-        long long r = e / m;
-        int col = (int)(e - r * m);
-        int l = col / m16, c = col - l * m16;
-        vperm[e] = v[r * m + 16 * c + l];
+        const long long r = e / m;
+        const int o = (int)(e - r * m);
+        const int s = o / rw, i = o - s * rw;  // lane pair in visiting order, position in it
+        const int l = (((s & 1) << 2) | (s & 2) | (s >> 2)) + 8 * (i & 1);
+        vperm[e] = v[r * m + 16 * (i >> 1) + l];
     }
 }
 

@@ -246,8 +246,9 @@ CT_API int ct_knn_residual_points(ct_tree* tree, const float* qv, const float* q
  *   ct_batch_add_ids     a query set of dataset ids (same contract as ct_knn_residual,
  *                        CT_FORM_DENSE: bit-identical output)
  *   ct_batch_add_points  a query set of new points (same contract as ct_knn_residual_points)
- *   ct_batch_set_shape   fix the launch shape: qt (queries per CTA tile: 16/32/64),
- *                        ctas_per_sm (1/2), items_per_slot (candidate-split target); 0 = auto
+ *   ct_batch_set_shape   fix the launch shape: qt (queries per CTA tile: 16 or 32; 64 runs as
+ *                        32-row tiles), ctas_per_sm (1/2; 1 where two do not fit),
+ *                        items_per_slot (candidate-split target); 0 = auto
  *   ct_batch_autotune    time the candidate shapes on the current batch (reps runs each,
  *                        synchronising `stream`) and keep the fastest
  *   ct_batch_run         launch every added query set; asynchronous on `stream`
