@@ -315,6 +315,7 @@ int ct_knn_euclidean(const float* points, int64_t n, int32_t d, const float* que
     if (d <= 0 || d > ct::euclid_max_d()) return fail(CT_ERR_UNSUPPORTED, "ct_knn_euclidean: d=%d outside [1, %d]", d, ct::euclid_max_d());
     if (nq == 0) return CT_OK;
     if (!points || !queries || !out_idx || !out_dist) return fail(CT_ERR_ARG, "ct_knn_euclidean: NULL pointer");
+    keep_pool_memory();
     CT_CUDA(ct::launch_euclid_knn(points, n, d, queries, nq, k, predecessor ? 1 : 0, (long long*)out_idx, out_dist,
                                   (cudaStream_t)stream), "euclidean kNN launch");
     return CT_OK;

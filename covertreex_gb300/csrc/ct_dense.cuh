@@ -298,7 +298,8 @@ static __device__ __noinline__ void merge_buffer(u64* list, int k, const u64* bu
 // Merge S sorted partial lists of k keys (list s at part + s * k) into out_* (one query by nw
 // warps of the block, this one their part_w-th; every thread of the block calls).  Lists whose
 // head does not beat the current k-th are skipped.  scratch: k keys of shared memory per warp.
-template <int E>
+// SQRT: the keys hold squared distances.
+template <int E, bool SQRT>
 __device__ __forceinline__ void merge_lists_e(const u64* part, int S, int k, int part_w, int nw, u64* scratch,
                                               bool active, long long* out_idx, float* out_dist) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -336,7 +337,8 @@ __device__ __forceinline__ void merge_lists_e(const u64* part, int S, int k, int
             const int j = e * 32 + lane;
             if (j < k) {
                 out_idx[j] = a[e] == kNoKey ? -1LL : (long long)(unsigned)a[e];
-                out_dist[j] = a[e] == kNoKey ? CT_FLT_MAX : __uint_as_float((unsigned)(a[e] >> 32));
+                const float v = __uint_as_float((unsigned)(a[e] >> 32));
+                out_dist[j] = a[e] == kNoKey ? CT_FLT_MAX : SQRT ? sqrtf(v) : v;
             }
         }
     }
@@ -344,7 +346,7 @@ __device__ __forceinline__ void merge_lists_e(const u64* part, int S, int k, int
 }
 // Final merge of a query tile by NT threads: queries [g0, g0 + nv), partial lists [query][S][k].
 // Fewer queries than warps get several warps each.
-template <int NT>
+template <int NT, bool SQRT = false>
 __device__ inline void merge_tile(const u64* part, int S, int k, long long g0, int nv, u64* scratch,
                                   long long* out_idx, float* out_dist, long long out_stride) {
     int nw = 1;
@@ -357,9 +359,9 @@ __device__ inline void merge_tile(const u64* part, int S, int k, long long g0, i
         const u64* src = part + (size_t)g * S * k;
         long long* oi = out_idx + g * out_stride;
         float* od = out_dist + g * out_stride;
-        if (k <= 32) merge_lists_e<1>(src, S, k, warp % nw, nw, scratch, active, oi, od);
-        else if (k <= 64) merge_lists_e<2>(src, S, k, warp % nw, nw, scratch, active, oi, od);
-        else merge_lists_e<4>(src, S, k, warp % nw, nw, scratch, active, oi, od);
+        if (k <= 32) merge_lists_e<1, SQRT>(src, S, k, warp % nw, nw, scratch, active, oi, od);
+        else if (k <= 64) merge_lists_e<2, SQRT>(src, S, k, warp % nw, nw, scratch, active, oi, od);
+        else merge_lists_e<4, SQRT>(src, S, k, warp % nw, nw, scratch, active, oi, od);
     }
 }
 
