@@ -3,16 +3,17 @@
 // without the budget ladder), exact: it returns the dense form's neighbour lists
 // bit for bit.
 //
-// One warp owns one query (persistent grid, queries strided over warps).  The warp
-// keeps its top-k (distance, dataset id) list sorted in shared memory and a
-// depth-first stack of (node, bound) in shared memory.  Candidate lists (the roots,
-// then the children of each expanded node) are filtered 32 at a time with a ballot
-// (predecessor mode: a subtree whose minimum dataset id is not below the query's is
-// skipped without a distance, src/algo.rs:900-916), and the surviving candidates are
-// scored 4 at a time: their V rows are staged in shared memory with 16-byte cp.async
-// copies, then each half-warp scores 2 rows with the reference's batch-path f32
-// distance (lane l sums elements 16c + l, bit-identical to the dense form) against
-// the query row held in registers.
+// One block owns one query at a time (persistent grid).  It keeps a depth-first stack of frames
+// (a range of child indices and the subtree's bound) and its top-k list in shared memory and
+// works in steps of kB candidates: the topmost frames' children (the roots when the stack is
+// empty) are gathered, filtered in predecessor mode (a subtree whose minimum dataset id is not
+// below the query's is skipped without a distance, src/algo.rs:900-916), their V rows scored by
+// half-warps with the reference's batch-path f32 distance (lane l sums elements 16c + l,
+// bit-identical to the dense form) and each candidate's normalisation, list key, bound and
+// children looked up by a thread of its own.  Candidates that have children and are not pruned
+// become frames.  A step costs a handful of dependent memory latencies whatever its width, so
+// its width is what sets the rate while the tree fits in L2: N = 16384, m = 128, 256 queries
+// 16.4 ms with a warp per query scoring 4 candidates at a time, 1.0 ms now.
 //
 // Prune (certified, ct_treebound.cuh): the subtree below a node a cannot hold a
 // neighbour when
@@ -25,7 +26,10 @@
 // has d32(q, x) > kth, so the pruned subtree cannot change the list: the result equals
 // the dense form's.  The reference's own test, d(q, a) - max(si[a], 1e-3) > kth on
 // FP32 values (src/algo.rs:814-818, 1113-1142), has no such guarantee.
+#include <algorithm>
+
 #include "ct_common.cuh"
+#include "ct_dense.cuh"
 #include "ct_internal.h"
 #include "ct_tree.h"
 #include "ct_treebound.cuh"
@@ -33,13 +37,16 @@
 namespace ct {
 namespace trav {
 
-constexpr int kWarps = 8;
-constexpr int kChunk = 8;                    // list entries a frame hands out per step
-// per tree level the stack holds at most one chunk's children; 40 levels (levels fall strictly
-// from 0 to -30, and only duplicate points share the floor level)
-constexpr int kStack = kChunk * 40 + 1;
+constexpr int kThreads = 256;
+constexpr int kB = 128;  // candidates of a step
+// A step pushes at most kB frames, and only the topmost batch of frames is consumed while it
+// lasts, so the batches on the stack have strictly growing least depths: kB frames per level of
+// the tree at most (levels fall strictly from 0 to -30; only duplicate points share the floor
+// level).  A deeper tree is reported as an overflow error, never written past.
+constexpr int kStack = kB * 40;
 constexpr int kTopK = 64;
-constexpr int kRows = 4;  // candidate rows staged per batch (2 per half-warp)
+constexpr int kBufKeep = 64;            // keys a step may leave unmerged
+constexpr int kBuf = kB + kBufKeep;
 
 struct Params {
     const float* v;      // node-order natural V
@@ -68,189 +75,210 @@ struct Params {
     int* overflow;
 };
 
-// Insert (d, id) into the warp's sorted top-k list if it beats the k-th entry.
-__device__ __forceinline__ void topk_offer(float* td, int* ti, int& cnt, int k, float d, int id) {
-    const int lane = threadIdx.x & 31;
-    const bool full = cnt >= k;
-    if (full && !nb_less(d, id, td[k - 1], ti[k - 1])) return;
-    int below = 0;
-    for (int j = lane; j < cnt; j += 32) below += nb_less(td[j], ti[j], d, id) ? 1 : 0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) below += __shfl_xor_sync(0xffffffffu, below, off);
-    const int last = full ? k - 1 : cnt;  // entries [below, last) shift right by one
-    float sd[2];
-    int si2[2];
-    int ns = 0;
-    for (int j = below + lane; j < last; j += 32) { sd[ns] = td[j]; si2[ns] = ti[j]; ++ns; }
-    __syncwarp();
-    ns = 0;
-    for (int j = below + lane; j < last; j += 32) { td[j + 1] = sd[ns]; ti[j + 1] = si2[ns]; ++ns; }
-    __syncwarp();
-    if (lane == 0) { td[below] = d; ti[below] = id; }
-    __syncwarp();
-    if (!full) ++cnt;
-}
+struct Frame {
+    int beg, end;  // child_idx range still to visit
+    float lb;      // certified lower bound of every FP32 distance below it
+};
+struct Shared {
+    Frame stack[kStack];
+    dense::u64 list[kTopK];
+    dense::u64 buf[kBuf];
+    int cand[kB];
+    float dot[kB];
+    float xq[64];
+    int fbeg[kB], ffirst[kB];  // the frames of a step: first child index, first candidate
+    int wsum[kThreads / 32];
+    int ncand, nframes, cnt, sp, overflow;
+    dense::u64 tau;
+};
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc));
-}
-
-template <int MAXC>
-__global__ void __launch_bounds__(32 * kWarps) traverse_kernel(Params P) {
+__global__ void __launch_bounds__(kThreads) traverse_kernel(Params P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_node[kWarps][kStack];
-    __shared__ int s_cur[kWarps][kStack];
-    __shared__ float s_lb[kWarps][kStack];
-    __shared__ float s_td[kWarps][kTopK];
-    __shared__ int s_ti[kWarps][kTopK];
-    __shared__ float s_xq[kWarps][64];
-    __shared__ int s_cand[kWarps][32];
-    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int half = (lane >> 4) & 1, l16 = lane & 15;
-    const unsigned hmask = half ? 0xffff0000u : 0x0000ffffu;
-    const long long nwarps = (long long)gridDim.x * kWarps;
-    const int m = P.m, mc = P.m >> 4;
-    float* rows = (float*)smem_raw + (size_t)wi * kRows * m;
-    int* stn = s_node[wi];
-    int* stc = s_cur[wi];
-    float* stl = s_lb[wi];
-    float* td = s_td[wi];
-    int* ti = s_ti[wi];
-    float* xq = s_xq[wi];
-    int* cand = s_cand[wi];
+    Shared& S = *(Shared*)smem_raw;
+    float* vq = (float*)(smem_raw + ((sizeof(Shared) + 15) & ~size_t(15)));  // query row
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int l16 = lane & 15, hw = tid >> 4;
+    const unsigned hmask = (lane & 16) ? 0xffff0000u : 0x0000ffffu;
+    const int m = P.m, mc = P.m >> 4, k = P.k;
     unsigned long long evals = 0;
-    for (long long qi = (long long)blockIdx.x * kWarps + wi; qi < P.nq; qi += nwarps) {
+    for (long long qi = blockIdx.x; qi < P.nq; qi += gridDim.x) {
         const long long qd = P.q_ids[qi];
-        int cnt = 0;
-        if (qd >= 0 && qd < P.n && !(P.predecessor && qd == 0)) {
-            const int qn = (int)P.inv[qd];
-            float vq[MAXC];
-#pragma unroll
-            for (int c = 0; c < MAXC; ++c) vq[c] = c < mc ? P.v[(size_t)qn * m + 16 * c + l16] : 0.f;
-            for (int c = lane; c < P.d; c += 32) xq[c] = P.xs[(size_t)qn * P.d + c];
-            const float nq = P.norms[qn], pq = P.p[qn], isq = P.isp[qn], vnq = P.vn[qn];
-            const bool may_prune = isq <= kNoPruneIsp;
-            bool overflowed = false;
-            // Depth-first over frames (node, cursor, bound): node -1 is the list of roots.
-            // A frame hands out its candidates kChunk at a time; expandable candidates
-            // become frames on top of it, so the stack holds at most kChunk frames per tree
-            // level; a deeper tree is reported as an overflow error, never read past.
-            int sp = 0;
-            if (lane == 0) { stn[0] = -1; stc[0] = 0; stl[0] = 0.f; }
-            sp = 1;
-            __syncwarp();
-            while (sp > 0) {
-                const int top = sp - 1;
-                const int nd = stn[top];
-                const int cur = stc[top];
-                const float lbf = stl[top];
-                __syncwarp();
-                const long long b0 = nd < 0 ? 0 : P.child_off[nd];
-                const long long e0 = nd < 0 ? P.n_roots : P.child_off[nd + 1];
-                const long long* ids = nd < 0 ? P.roots : P.child_idx;
-                const float kth0 = cnt >= P.k ? td[P.k - 1] : CT_FLT_MAX;
-                const long long base = b0 + cur;
-                if (base >= e0 || lbf > kth0) {  // frame done, or its whole subtree pruned
-                    --sp;
-                    continue;
+        const bool live = qd >= 0 && qd < P.n && !(P.predecessor && qd == 0);
+        __syncthreads();  // the previous query's results have been written
+        for (int j = tid; j < k; j += kThreads) S.list[j] = dense::kNoKey;
+        if (tid == 0) { S.cnt = 0; S.sp = 0; S.tau = dense::kNoKey; S.overflow = 0; }
+        const int qn = live ? (int)P.inv[qd] : 0;
+        if (live) {
+            for (int c = tid; c < m; c += kThreads) vq[c] = P.v[(size_t)qn * m + c];
+            for (int c = tid; c < P.d; c += kThreads) S.xq[c] = P.xs[(size_t)qn * P.d + c];
+        }
+        const float nq = P.norms[qn], pq = P.p[qn], isq = P.isp[qn], vnq = P.vn[qn];
+        const bool may_prune = isq <= kNoPruneIsp;
+        long long next_root = live ? 0 : P.n_roots;
+        __syncthreads();
+        for (;;) {
+            // ---- gather up to kB candidates from the topmost frames, or from the roots
+            const int sp = S.sp;
+            if (sp == 0 && next_root >= P.n_roots) break;
+            const dense::u64 tau = S.tau;
+            const float kth = tau == dense::kNoKey ? CT_FLT_MAX : __uint_as_float((unsigned)(tau >> 32));
+            int c = -1;
+            int total;
+            if (sp == 0) {
+                const long long left = P.n_roots - next_root;
+                total = left < kB ? (int)left : kB;
+                if (tid < total) c = (int)P.roots[next_root + tid];
+                next_root += total;
+                __syncthreads();  // every thread has read the stack state
+            } else {
+                // thread i looks at the i-th frame from the top; a pruned frame offers nothing
+                int take = 0;
+                Frame f{0, 0, 0.f};
+                if (tid < kB && tid < sp) {
+                    f = S.stack[sp - 1 - tid];
+                    take = f.lb > kth ? 0 : min(f.end - f.beg, kB);
                 }
-                if (lane == 0) stc[top] = cur + kChunk;
-                const long long gi = base + lane;
-                int c = (lane < kChunk && gi < e0) ? (int)ids[gi] : -1;
-                if (c >= 0 && P.predecessor && P.sub_min[c] >= qd) c = -1;
-                const unsigned ok = __ballot_sync(0xffffffffu, c >= 0);
-                if (c >= 0) cand[__popc(ok & ((1u << lane) - 1u))] = c;
-                __syncwarp();
-                const int nc = __popc(ok);
-                for (int c0 = 0; c0 < nc; c0 += kRows) {
-                    const int nr = min(kRows, nc - c0);
-                    // stage nr rows: 16-byte pieces spread over the warp
-                    const int pieces = m >> 2;  // per row
-                    for (int t = lane; t < nr * pieces; t += 32) {
-                        const int r = t / pieces, q4 = t - r * pieces;
-                        cp_async16(rows + (size_t)r * m + 4 * q4, P.v + (size_t)cand[c0 + r] * m + 4 * q4);
-                    }
-                    asm volatile("cp.async.commit_group;\n" ::);
-                    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-                    __syncwarp();
-                    float dist[kRows / 2];
+                int incl = take;
 #pragma unroll
-                    for (int r = 0; r < kRows / 2; ++r) {
-                        const int rr = half * (kRows / 2) + r;
-                        dist[r] = CT_FLT_MAX;
-                        if (rr < nr) {
-                            const float* row = rows + (size_t)rr * m;
-                            float acc = 0.f;
-#pragma unroll
-                            for (int cc = 0; cc < MAXC; ++cc)
-                                if (cc < mc) acc = __fadd_rn(__fmul_rn(vq[cc], row[16 * cc + l16]), acc);
-                            float t = __shfl_down_sync(hmask, acc, 8, 16);
-                            const float comb = __fadd_rn(acc, t);
-                            t = __shfl_down_sync(hmask, comb, 4, 16);
-                            const float s2 = __fadd_rn(comb, t);
-                            t = __shfl_down_sync(hmask, s2, 2, 16);
-                            const float u2 = __fadd_rn(s2, t);
-                            t = __shfl_down_sync(hmask, u2, 1, 16);
-                            float dot = __fadd_rn(u2, t);
-                            dot = __shfl_sync(hmask, dot, 0, 16);
-                            const int node = cand[c0 + rr];
-                            if (node == qn) {
-                                dist[r] = 0.f;
-                            } else {
-                                const float d2 = coord_d2_batch(xq, P.xs + (size_t)node * P.d, P.d, nq, P.norms[node]);
-                                const float kv = kernel_value_batch(d2, P.var, P.kernel_type);
-                                dist[r] = residual_from_parts(kv, dot, pq, P.p[node]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int rr = 0; rr < kRows; ++rr) {
-                        if (rr < nr) {
-                            const float dd = __shfl_sync(0xffffffffu, dist[rr % (kRows / 2)], rr < kRows / 2 ? 0 : 16);
-                            const int node = cand[c0 + rr];
-                            const long long ds = P.order[node];
-                            ++evals;
-                            if (!P.predecessor || ds < qd) topk_offer(td, ti, cnt, P.k, dd, (int)ds);
-                            if (P.child_off[node + 1] > P.child_off[node]) {
-                                float lb = 0.f;
-                                if (may_prune) {
-                                    const float dqa = pair_delta(P.bound, nq, P.norms[node], vnq, P.vn[node], isq,
-                                                                 P.isp[node]);
-                                    const float L = (dist_lower(dd, dqa) - P.si_up[node]) * (1.f - 5.0e-7f);
-                                    if (L > 0.f) {
-                                        const float dmax = pair_delta(P.bound, nq, P.bound.nmax, vnq, P.bound.vmax,
-                                                                      isq, P.sub_isp[node]);
-                                        lb = dist_lower(L, dmax);
-                                    }
-                                }
-                                const float kth = cnt >= P.k ? td[P.k - 1] : CT_FLT_MAX;
-                                if (!(lb > kth)) {
-                                    if (sp < kStack) {
-                                        if (lane == 0) { stn[sp] = node; stc[sp] = 0; stl[sp] = lb; }
-                                        ++sp;
-                                    } else {
-                                        overflowed = true;
-                                    }
-                                }
-                            }
-                            __syncwarp();
-                        }
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (lane == 31) S.wsum[warp] = incl;
+                __syncthreads();
+                for (int w = 0; w < warp; ++w) incl += S.wsum[w];
+                const int first = incl - take;  // candidates of the frames above this one
+                // frames wholly or partly taken: those whose first candidate lies below kB
+                if (tid < kB && tid < sp && first < kB) {
+                    S.fbeg[tid] = f.beg;
+                    S.ffirst[tid] = first;
+                    const bool part = first + take > kB;
+                    const bool last = tid + 1 == min(sp, kB) || incl >= kB;
+                    if (part) S.stack[sp - 1 - tid].beg = f.beg + (kB - first);
+                    if (last) {  // the deepest frame of the step
+                        S.nframes = tid + 1;
+                        S.ncand = min(incl, kB);
+                        // a frame with children left stays, the ones above it go
+                        const bool stays = part || (first + take == kB && f.lb <= kth && f.end - f.beg > take);
+                        if (!part && stays) S.stack[sp - 1 - tid].beg = f.beg + take;
+                        S.sp = sp - tid - (stays ? 0 : 1);
                     }
                 }
-                __syncwarp();
+                __syncthreads();
+                total = S.ncand;
+                if (tid < total) {
+                    int lo = 0, hi = S.nframes - 1;  // last frame whose first candidate is <= tid
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (S.ffirst[mid] <= tid) lo = mid; else hi = mid - 1;
+                    }
+                    c = (int)P.child_idx[S.fbeg[lo] + (tid - S.ffirst[lo])];
+                }
             }
-            if (overflowed && lane == 0) atomicAdd(P.overflow, 1);
+            if (c >= 0 && P.predecessor && P.sub_min[c] >= qd) c = -1;
+            // compact
+            const unsigned okm = __ballot_sync(0xffffffffu, c >= 0);
+            if (lane == 0) S.wsum[warp] = __popc(okm);
+            __syncthreads();
+            int at = __popc(okm & ((1u << lane) - 1u)), nc = 0;
+            for (int w = 0; w < kThreads / 32; ++w) {
+                if (w < warp) at += S.wsum[w];
+                nc += S.wsum[w];
+            }
+            if (c >= 0) S.cand[at] = c;
+            __syncthreads();
+            // ---- V dots: half-warp h scores candidates h, h + 16, ..., four rows in flight
+            for (int c0 = hw; c0 < nc; c0 += 64) {
+                const float* row[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) row[u] = P.v + (size_t)S.cand[c0 + 16 * u < nc ? c0 + 16 * u : c0] * m + l16;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+                for (int cc = 0; cc < mc; ++cc) {
+                    const float a = vq[16 * cc + l16];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc[u] = __fadd_rn(__fmul_rn(a, __ldg(row[u] + 16 * cc)), acc[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float t = __shfl_down_sync(hmask, acc[u], 8, 16);
+                    const float comb = __fadd_rn(acc[u], t);
+                    t = __shfl_down_sync(hmask, comb, 4, 16);
+                    const float s2 = __fadd_rn(comb, t);
+                    t = __shfl_down_sync(hmask, s2, 2, 16);
+                    const float u2 = __fadd_rn(s2, t);
+                    t = __shfl_down_sync(hmask, u2, 1, 16);
+                    if (l16 == 0 && c0 + 16 * u < nc) S.dot[c0 + 16 * u] = __fadd_rn(u2, t);
+                }
+            }
+            __syncthreads();
+            // ---- one candidate per thread: distance, list, bound, children
+            bool push = false;
+            Frame f{0, 0, 0.f};
+            if (tid < nc) {
+                const int node = S.cand[tid];
+                const long long ds = P.order[node];
+                const long long b0 = P.child_off[node], e0 = P.child_off[node + 1];
+                const float nn = P.norms[node];
+                float dist = 0.f;
+                if (node != qn) {
+                    const float d2 = coord_d2_batch(S.xq, P.xs + (size_t)node * P.d, P.d, nq, nn);
+                    const float kv = kernel_value_batch(d2, P.var, P.kernel_type);
+                    dist = residual_from_parts(kv, S.dot[tid], pq, P.p[node]);
+                }
+                if (!P.predecessor || ds < qd) {
+                    const dense::u64 key = dense::make_key(dist, (int)ds);
+                    if (key < tau) S.buf[atomicAdd(&S.cnt, 1)] = key;
+                }
+                if (e0 > b0) {
+                    f.beg = (int)b0;
+                    f.end = (int)e0;
+                    if (may_prune) {
+                        const float dqa = pair_delta(P.bound, nq, nn, vnq, P.vn[node], isq, P.isp[node]);
+                        const float L = (dist_lower(dist, dqa) - P.si_up[node]) * (1.f - 5.0e-7f);
+                        if (L > 0.f) {
+                            const float dmax = pair_delta(P.bound, nq, P.bound.nmax, vnq, P.bound.vmax, isq,
+                                                          P.sub_isp[node]);
+                            f.lb = dist_lower(L, dmax);
+                        }
+                    }
+                    push = !(f.lb > kth);
+                }
+            }
+            evals += nc;
+            const unsigned pm = __ballot_sync(0xffffffffu, push);
+            if (lane == 0) S.wsum[warp] = __popc(pm);
+            __syncthreads();
+            const int sp0 = S.sp;
+            int pos = sp0 + __popc(pm & ((1u << lane) - 1u)), np = 0;
+            for (int w = 0; w < kThreads / 32; ++w) {
+                if (w < warp) pos += S.wsum[w];
+                np += S.wsum[w];
+            }
+            if (push && pos < kStack) S.stack[pos] = f;
+            const int cnt = S.cnt;
+            __syncthreads();
+            if (tid == 0) {
+                S.sp = min(sp0 + np, kStack);
+                if (sp0 + np > kStack) S.overflow = 1;
+            }
+            if (warp == 1 && cnt > kBufKeep) {
+                dense::merge_buffer(S.list, k, S.buf, cnt);
+                if (lane == 0) { S.cnt = 0; S.tau = S.list[k - 1]; }
+            }
+            __syncthreads();
         }
-        for (int j = lane; j < P.k; j += 32) {
-            const bool ok = j < cnt;
-            P.out_idx[qi * P.k + j] = ok ? (long long)ti[j] : -1LL;
-            P.out_dist[qi * P.k + j] = ok ? td[j] : CT_FLT_MAX;
+        if (warp == 0) {
+            dense::merge_buffer(S.list, k, S.buf, S.cnt);
+            for (int j = lane; j < k; j += 32) {
+                const dense::u64 key = S.list[j];
+                P.out_idx[qi * k + j] = key == dense::kNoKey ? -1LL : (long long)(unsigned)key;
+                P.out_dist[qi * k + j] = key == dense::kNoKey ? CT_FLT_MAX : __uint_as_float((unsigned)(key >> 32));
+            }
+            if (lane == 0 && S.overflow) atomicAdd(P.overflow, 1);
         }
-        __syncwarp();
     }
-    if (lane == 0 && P.evals) atomicAdd(P.evals, evals);
+    if (tid == 0 && P.evals && evals) atomicAdd(P.evals, evals);
 }
 
 }  // namespace trav
@@ -279,20 +307,14 @@ int ct_tree::knn_tree(const int64_t* q_ids, int64_t nq, int k, int predecessor, 
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = sizeof(float) * (size_t)kWarps * kRows * m;
-    long long blocks = (nq + kWarps - 1) / kWarps;
-    if (blocks > (long long)sms * 16) blocks = (long long)sms * 16;
+    const size_t smem = ((sizeof(Shared) + 15) & ~size_t(15)) + sizeof(float) * (size_t)m;
+    const long long blocks = std::min<long long>(nq, (long long)sms * 3);  // three blocks' stacks fit an SM
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     const bool timing = ct::timing_enabled();
     if (timing) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, st); }
     if (e == cudaSuccess) {
-        if (m <= 512) {
-            e = cudaFuncSetAttribute(traverse_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e == cudaSuccess) traverse_kernel<32><<<(unsigned)blocks, 32 * kWarps, smem, st>>>(P);
-        } else {
-            e = cudaFuncSetAttribute(traverse_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e == cudaSuccess) traverse_kernel<64><<<(unsigned)blocks, 32 * kWarps, smem, st>>>(P);
-        }
+        e = cudaFuncSetAttribute(traverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) traverse_kernel<<<(unsigned)blocks, kThreads, smem, st>>>(P);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     unsigned long long he = 0;
