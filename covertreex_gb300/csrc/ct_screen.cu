@@ -130,9 +130,10 @@ struct MMAParams {
     int parts;           // candidate parts per query (slots s*parts .. s*parts+parts-1)
 };
 
+constexpr int kUnionEvery = 16;  // kept jobs between two row_kth calls
 constexpr int kRing = 4;  // claimed units in flight per CTA (dynamic schedule)
 struct SmemLayout {
-    size_t stages, rec, heap, rowtau, bars, tmem_slot, ring, total;
+    size_t stages, rec, heap, rowtau, hcnt, bars, tmem_slot, ring, total;
 };
 __host__ __device__ inline SmemLayout smem_layout(int k, int nstages) {
     SmemLayout L;
@@ -141,7 +142,8 @@ __host__ __device__ inline SmemLayout smem_layout(int k, int nstages) {
     L.rec = off; off += (size_t)2 * RT * sizeof(float);
     L.heap = off; off += (size_t)kEpiThreads * (k > 0 ? k : 1) * sizeof(float);
     L.rowtau = off; off += (size_t)TQ * sizeof(unsigned long long);
-    L.bars = off; off += (size_t)(2 * STAGES + 4 + 4 + 1 + 2 * kRing) * 8;
+    L.hcnt = off; off += (size_t)kEpiThreads * sizeof(int);
+    L.bars = off; off += (size_t)(2 * STAGES + 4 + 4 + 1 + 2 * kRing + 4) * 8;
     L.tmem_slot = off; off += 16;
     L.ring = off; off += 16;
     L.total = off + 1024;  // alignment slack
@@ -185,8 +187,29 @@ __device__ __forceinline__ void heap_push(float* h, int n, float x) {
     h[i * kEpiThreads] = x;
 }
 
-// bit 2 of `which`: a kept job whose candidate tile already fed the heap during warm-up
-__device__ __forceinline__ bool jb_warm_seen(const Job& jb) { return (jb.which & 4) != 0; }
+// e^x as ex2.approx of x log2(e), results below 2^-126 flushed to zero (__expf's own two steps without
+// its scaling of tiny results, whose 1e-38 the bounds' absolute 1e-30 covers).
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float2 exp2x(float2 x) {
+    const float2 t = __fmul2_rn(x, make_float2(1.4426950408889634f, 1.4426950408889634f));
+    return make_float2(ex2_ftz(t.x), ex2_ftz(t.y));
+}
+// sqrt(x), x >= 0: s = x rsqrt(x) and one correction step, within 2^-45 relative before its last
+// rounding (half an ulp, as the bounds assume), without the branches of the IEEE routine.
+// 1e-15 for x = 0.
+__device__ __forceinline__ float2 sqrt2x(float2 x) {
+    x = make_float2(fmaxf(x.x, 1e-30f), fmaxf(x.y, 1e-30f));
+    float2 r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+    const float2 s = __fmul2_rn(x, r);
+    const float2 e = __ffma2_rn(make_float2(-s.x, -s.y), s, x);
+    return __ffma2_rn(e, __fmul2_rn(r, make_float2(0.5f, 0.5f)), s);
+}
 
 // Squared scaled distance and kernel value of one query with two staged candidates
 // (columns .x and .y of the record pair r4).  Matern also returns a = sqrt(5 d2) and e^-a
@@ -206,11 +229,11 @@ __device__ __forceinline__ void pair_kv2(const float4* r4, const float (&nxq)[kM
     }
     if (KT == 0) {
         const float2 h = __fmul2_rn(make_float2(-0.5f, -0.5f), d2);
-        kv = __fmul2_rn(make_float2(var, var), make_float2(__expf(h.x), __expf(h.y)));
+        kv = __fmul2_rn(make_float2(var, var), exp2x(h));
         a = ea = make_float2(0.f, 0.f);
     } else {
-        a = __fmul2_rn(make_float2(2.2360679775f, 2.2360679775f), make_float2(sqrtf(d2.x), sqrtf(d2.y)));
-        ea = make_float2(__expf(-a.x), __expf(-a.y));
+        a = __fmul2_rn(make_float2(2.2360679775f, 2.2360679775f), sqrt2x(d2));
+        ea = exp2x(make_float2(-a.x, -a.y));
         // var (1 + a + a^2 / 3) e^-a, each step rounded
         const float2 a2 = __fmul2_rn(__fmul2_rn(a, a), make_float2(0.33333334f, 0.33333334f));
         const float2 poly = __fadd2_rn(__fadd2_rn(make_float2(1.f, 1.f), a), a2);
@@ -223,7 +246,8 @@ __device__ __forceinline__ void pair_kv2(const float4* r4, const float (&nxq)[kM
 template <int MODE, int DP, int KT>
 __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    // (offset from smem_raw, so that the compiler keeps these shared-memory accesses, not generic ones)
+    unsigned char* smem = smem_raw + ((1024u - (sm::smem_u32(smem_raw) & 1023u)) & 1023u);
     const SmemLayout L = smem_layout(P.k, P.nstages);
     const int NS = P.nstages;
     unsigned char* stage_base = smem + L.stages;
@@ -239,6 +263,8 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
     uint64_t* done = rece + 2;
     uint64_t* rfull = done + 1;        // unit ring: slot written by the producer
     uint64_t* rempty = rfull + kRing;  // slot released by every consumer
+    uint64_t* pairb = rempty + kRing;  // the two epilogue warps of a row quarter
+    int* hcnt = (int*)(smem + L.hcnt);  // heap fill per epilogue thread (row_kth)
     uint32_t* tmem_slot = (uint32_t*)(smem + L.tmem_slot);
     int* ring = (int*)(smem + L.ring);
 
@@ -259,6 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
             sm::mbar_init(&rfull[r], 1);
             sm::mbar_init(&rempty[r], MODE == MODE_SWEEP ? 2 + kEpiWarps : 1 + kEpiWarps);
         }
+        for (int r = 0; r < 4; ++r) sm::mbar_init(&pairb[r], 2);
         sm::fence_barrier_init();
     }
     for (int r = threadIdx.x; r < TQ; r += blockDim.x) rowtau[r] = 0ULL;
@@ -437,6 +464,53 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
         const float dd = (float)P.d;
         const float ced2 = (dd + 2.f) * 5.97e-8f;
         bool alive = true;
+        auto set_tau = [&](float t) {
+            tau2 = t;
+            thr_keep = (1.f - tau2) * (1.f - 2e-6f) / isq;
+            thr_heap = (1.f - tau2) * (1.f + 2e-6f) / isq;
+        };
+        unsigned pair_phase = 0;
+        auto pair_sync = [&]() -> bool {
+            __syncwarp();
+            if (lane == 0) sm::mbar_arrive(&pairb[quarter]);
+            const bool ok = sm::mbar_wait(&pairb[quarter], pair_phase, P.status, 20);
+            pair_phase ^= 1u;
+            return ok;
+        };
+        // The row's threshold from both halves' heaps.  A half's own k-th bound is about the row's
+        // 2k-th; the k smallest bounds of the row all lie in its two heaps, so the k-th of their union
+        // (found from above by bisection, an upper bound whenever it stops) bounds the row's k-th
+        // distance.  Both warps of the row quarter call it at the same jobs; the heaps rest between
+        // the two pair barriers.
+        auto row_kth = [&]() -> bool {
+            hcnt[et] = hn;
+            if (!pair_sync()) return false;
+            const int hp = hcnt[et ^ 128];
+            const float* ph = heaps + (et ^ 128);
+            if (qid >= 0 && !ovf && hn + hp >= P.k) {
+                float lo = 0.f, hi = tau2;
+                if (hn >= P.k) hi = fminf(hi, heap[0]);
+                if (hp >= P.k) hi = fminf(hi, ph[0]);
+                auto count = [&](float t) {
+                    int c = 0;
+                    for (int i = 0; i < hn; ++i) c += heap[i * kEpiThreads] <= t;
+                    for (int i = 0; i < hp; ++i) c += ph[i * kEpiThreads] <= t;
+                    return c;
+                };
+                if (count(hi) >= P.k) {
+                    for (int it = 0; it < 10; ++it) {
+                        const float mid = 0.5f * (lo + hi);
+                        if (count(mid) >= P.k) hi = mid; else lo = mid;
+                    }
+                    if (hi < tau2) {
+                        set_tau(hi);
+                        if (P.parts > 1) atomicMin(&P.qtau[slot / P.parts], __float_as_uint(tau2));
+                    }
+                }
+            }
+            return pair_sync();
+        };
+        bool prev_warm = false;
         for (int ui = 0; alive; ++ui) {
         int j0u, j1u;
         if (!take_unit(ui, j0u, j1u)) break;
@@ -444,6 +518,10 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
             const Job jb = P.jobs[j];
             const int acc = lt & 1;
             const unsigned aph = (unsigned)((lt >> 1) & 1);
+            if (MODE == MODE_SWEEP && !jb.first && !(jb.which & 2) && (prev_warm || ((j - j0u) & (kUnionEvery - 1)) == 0)) {
+                if (!row_kth()) { alive = false; break; }
+            }
+            prev_warm = (jb.which & 2) != 0;
             if (MODE == MODE_SWEEP && jb.first) {
                 if (slot >= 0) {
                     P.surv_cnt[2 * slot + half] = cnt;
@@ -513,20 +591,12 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
                 const unsigned long long w = *(volatile unsigned long long*)&rowtau[row];
                 if ((unsigned)(w >> 32) == gen) {
                     const float t = __uint_as_float(~(unsigned)w);
-                    if (t < tau2) {
-                        tau2 = t;
-                        thr_keep = (1.f - tau2) * (1.f - 2e-6f) / isq;
-                        thr_heap = (1.f - tau2) * (1.f + 2e-6f) / isq;
-                    }
+                    if (t < tau2) set_tau(t);
                 }
                 // the other parts' thresholds of this query (any part's k-th upper
                 // bound bounds the query's k-th distance)
                 const float tg = __uint_as_float(__ldcg(&P.qtau[slot / P.parts]));
-                if (tg < tau2) {
-                    tau2 = tg;
-                    thr_keep = (1.f - tau2) * (1.f - 2e-6f) / isq;
-                    thr_heap = (1.f - tau2) * (1.f + 2e-6f) / isq;
-                }
+                if (tg < tau2) set_tau(tg);
             }
             for (int cc = 0; cc < 16; ++cc) {
                 float v[8];
@@ -679,9 +749,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
                         if (changed) {
                             const float top = heap[0];
                             if (top < tau2) {
-                                tau2 = top;
-                                thr_keep = (1.f - tau2) * (1.f - 2e-6f) / isq;
-                                thr_heap = (1.f - tau2) * (1.f + 2e-6f) / isq;
+                                set_tau(top);
                                 atomicMax(&rowtau[row], ((unsigned long long)gen << 32) |
                                                             (unsigned long long)(~__float_as_uint(tau2)));
                                 if (P.parts > 1) atomicMin(&P.qtau[slot / P.parts], __float_as_uint(tau2));
@@ -697,6 +765,8 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
                 if (MODE == MODE_SWEEP) sm::mbar_arrive(&rece[acc]);
             }
         }
+        // the unit's final thresholds, for the survivor pass
+        if (MODE == MODE_SWEEP && alive && !row_kth()) alive = false;
         __syncwarp();
         if (lane == 0) release_unit(ui);
         }
@@ -1172,12 +1242,12 @@ __device__ __forceinline__ void pair_bounds_core(const RescoreParams& P, const f
     }
     float kv, ek;
     if (P.kernel_type == 0) {
-        kv = __fmul_rn(P.var, __expf(__fmul_rn(-0.5f, d2)));
+        kv = __fmul_rn(P.var, ex2_ftz(__fmul_rn(__fmul_rn(-0.5f, d2), 1.4426950408889634f)));
         ek = __fmul_rn(kv, __fmaf_rn(alk, d2, bek));
     } else {
         const float ed2 = __fmaf_rn(ale, d2, bee);
-        const float a = 2.2360679775f * sqrtf(d2);
-        const float ea = __expf(-a);
+        const float a = 2.2360679775f * sqrt2x(make_float2(d2, d2)).x;
+        const float ea = ex2_ftz(-a * 1.4426950408889634f);
         kv = P.var * (1.f + a + a * a * 0.33333334f) * ea;
         ek = kv * (1e-6f + 2.4e-7f * a) + P.var * (0.8334f * ed2 + 1e-7f * a * a) * (1.f + a) * ea;
     }
@@ -1475,7 +1545,11 @@ __global__ void inverse_perm_kernel(const int* order, long long n, int* inv) {
 // of the level's query range), low 32 bits = row of the query's Hilbert
 // position inside its level.  Queries without a level sort last.
 constexpr int kBands = 16;
-constexpr int kWarmTiles = 32;  // nearest candidate tiles that set the thresholds before any pair is kept (measured best of 8-64)
+// Nearest candidate tiles that set the thresholds before any pair is kept: 8, or 16 from levels of 256
+// tiles on.  Fewer leave loose thresholds and multiply the survivors, more repeat tiles whose heap
+// updates cost three times a kept job (measured: N=32768 7.3 ms at 8, 7.4 at 16, 7.9 at 32; N=262144
+// 147 ms at 8, 139.7 at 16, 141.5 at 32).
+constexpr int kWarmTiles = 8, kWarmTilesLarge = 16, kLargeLevel = 256;
 
 // A (query tile, part) unit of the sweep and the kernel that writes its jobs.
 struct JobUnit {
@@ -2633,7 +2707,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
             if (mine == 0) continue;
             const int nlev_mine = sp.ntl > pp ? (sp.ntl - pp + parts - 1) / parts : 0;
             // seeded queries start from a tight threshold: two warm-up tiles fill the heaps
-            const int warm_cap = seeded ? 2 : kWarmTiles;
+            const int warm_cap = seeded ? 2 : sp.ntl >= kLargeLevel ? kWarmTilesLarge : kWarmTiles;
             const int warm = std::min(parts > 1 ? std::max(1, std::min(warm_cap, nlev_mine / 4)) : warm_cap,
                                       nlev_mine);
             JobUnit u;
