@@ -813,14 +813,16 @@ __global__ void build_records_kernel(const int* __restrict__ ids, long long rows
 }
 
 // Half-tile boxes and group scalars of the sweep's group test (after a tile's candidate
-// records): one thread per half tile writes the box of its 128 candidates' scaled
+// records): a warp per half tile writes the box of its 128 candidates' scaled
 // coordinates (lo in floats 0-7, hi in 8-15; 0 past d; an empty box +inf / -inf when no
 // row is valid) and, for each of its 16 groups of 8, the largest err_coef |v| and the
-// largest 1/sqrt(p) (NaN when the group has no valid row).
+// largest 1/sqrt(p) (NaN when the group has no valid row).  Lane l takes candidates 4l .. 4l+3,
+// so a group is two lanes.
 __global__ void build_group_records_kernel(const int* __restrict__ ids, long long rows, const float* __restrict__ xs,
                                            int d, const float* __restrict__ vn, const float* __restrict__ isp,
                                            float err_coef, float* __restrict__ rec) {
-    const long long hi_ = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long hi_ = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (hi_ >= rows / (TC / 2)) return;
     const long long tile = hi_ / 2;
     const int h = (int)(hi_ - tile * 2);
@@ -828,28 +830,36 @@ __global__ void build_group_records_kernel(const int* __restrict__ ids, long lon
 #pragma unroll
     for (int c = 0; c < kMaxD; ++c) { lo[c] = __int_as_float(0x7f800000); hi[c] = -__int_as_float(0x7f800000); }
     float* base = rec + tile * RT + TC * REC;
-    for (int g = 0; g < TC / 16; ++g) {
-        float emax = 0.f, imax = __int_as_float(0x7fc00000);
-        bool any = false;
-        for (int e = 0; e < 8; ++e) {
-            const int cid = ids[tile * TC + h * (TC / 2) + 8 * g + e];
-            if (cid < 0) continue;
+    float emax = 0.f, imax = __int_as_float(0x7fc00000);  // (fmaxf passes a NaN by: NaN only without a valid row)
 #pragma unroll
-            for (int c = 0; c < kMaxD; ++c) {
-                const float x = c < d ? xs[(size_t)cid * d + c] : 0.f;
-                lo[c] = fminf(lo[c], x);
-                hi[c] = fmaxf(hi[c], x);
-            }
-            emax = fmaxf(emax, err_coef * vn[cid]);
-            imax = any ? fmaxf(imax, isp[cid]) : isp[cid];
-            any = true;
+    for (int e = 0; e < 4; ++e) {
+        const int cid = ids[tile * TC + h * (TC / 2) + 4 * lane + e];
+        if (cid < 0) continue;
+#pragma unroll
+        for (int c = 0; c < kMaxD; ++c) {
+            const float x = c < d ? xs[(size_t)cid * d + c] : 0.f;
+            lo[c] = fminf(lo[c], x);
+            hi[c] = fmaxf(hi[c], x);
         }
-        float* o = base + 2 * HBOX + (size_t)(h * (TC / 16) + g) * GREC;
+        emax = fmaxf(emax, err_coef * vn[cid]);
+        imax = fmaxf(imax, isp[cid]);
+    }
+    emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, 1));
+    imax = fmaxf(imax, __shfl_xor_sync(0xffffffffu, imax, 1));
+    if ((lane & 1) == 0) {
+        float* o = base + 2 * HBOX + (size_t)(h * (TC / 16) + (lane >> 1)) * GREC;
         o[0] = emax;
         o[1] = imax;
     }
 #pragma unroll
-    for (int c = 0; c < kMaxD; ++c) { base[h * HBOX + c] = lo[c]; base[h * HBOX + 8 + c] = hi[c]; }
+    for (int c = 0; c < kMaxD; ++c) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+            hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+        }
+        if (lane == 0) { base[h * HBOX + c] = lo[c]; base[h * HBOX + 8 + c] = hi[c]; }
+    }
 }
 
 // hi/lo split of V rows into the blocked layout.  rowmap[r] = dataset row of
@@ -879,15 +889,29 @@ __global__ void split_blocked_kernel(const float* __restrict__ v, int m, const i
     }
 }
 
-// vn = ||v|| rounded up, isp = 1/sqrt(p), xmax = max |xs|.
+// vn = ||v|| rounded up, isp = 1/sqrt(p), xmax = max |xs|.  A warp takes 32 rows: row by row it
+// sums the squares in FP32, every step rounded up (an upper bound of ||v|| within
+// (m / 32 + 5) 2^-23 of it), then each lane finishes a row (the FP64 reciprocal root of p costs a
+// warp as much for one lane as for 32).  65536 rows of 256: 12 us; 64 us as one strided FP64
+// chain per thread.
 __global__ void point_scalars_kernel(const float* __restrict__ v, const float* __restrict__ p,
                                      const float* __restrict__ xs, long long n, int m, int d, float* __restrict__ vn,
                                      float* __restrict__ isp, float* __restrict__ xmax) {
-    long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long r0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) & ~31LL;
+    const int lane = threadIdx.x & 31;
+    const int rows = r0 < n ? (int)(n - r0 < 32 ? n - r0 : 32) : 0;
+    float mine = 0.f;
+    for (int i = 0; i < rows; ++i) {
+        const float* row = v + (size_t)(r0 + i) * m;
+        float s = 0.f;
+        for (int c = lane; c < m; c += 32) s = __fmaf_ru(row[c], row[c], s);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = __fadd_ru(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (lane == i) mine = s;
+    }
+    const long long r = r0 + lane;
     if (r >= n) return;
-    double s = 0.0;
-    for (int c = 0; c < m; ++c) { double x = v[(size_t)r * m + c]; s += x * x; }
-    vn[r] = __double2float_ru(sqrt(s) * (1.0 + 1e-12));
+    vn[r] = __fsqrt_ru(mine);
     isp[r] = (float)(1.0 / sqrt((double)p[r]));
     float mx = 0.f;
     for (int c = 0; c < d; ++c) mx = fmaxf(mx, fabsf(xs[(size_t)r * d + c]));
@@ -1536,9 +1560,52 @@ __global__ void gather_ids_kernel(const int* order, long long n, long long rows,
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i < rows) out[i] = i < n ? order[i] : -1;
 }
-__global__ void inverse_perm_kernel(const int* order, long long n, int* inv) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) inv[order[i]] = (int)i;
+// Level rows: the Hilbert order filtered to ids < size (stable, so still key-sorted).  One block per
+// level walks the order kLevelItems rows per thread at a time; the padding rows keep the fill
+// (id -1, key ~0).
+constexpr int kLevelItems = 8;
+__global__ void __launch_bounds__(1024) build_levels_kernel(const int* __restrict__ order,
+                                                            const unsigned long long* __restrict__ key_by_id,
+                                                            long long n, const long long* __restrict__ meta,
+                                                            int* __restrict__ lvl_id,
+                                                            unsigned long long* __restrict__ lvl_key) {
+    __shared__ int wsum[32];
+    const long long size = meta[3 * blockIdx.x];
+    long long out = meta[3 * blockIdx.x + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (long long base = 0; base < n; base += 1024LL * kLevelItems) {
+        int id[kLevelItems];
+        int mine = 0;
+#pragma unroll
+        for (int e = 0; e < kLevelItems; ++e) {
+            const long long i = base + (long long)threadIdx.x * kLevelItems + e;
+            id[e] = i < n ? order[i] : 0x7fffffff;
+            mine += id[e] < size;
+        }
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int before = 0, total = 0;
+        for (int w = 0; w < 32; ++w) {
+            before += w < warp ? wsum[w] : 0;
+            total += wsum[w];
+        }
+        long long at = out + before + incl - mine;
+#pragma unroll
+        for (int e = 0; e < kLevelItems; ++e)
+            if (id[e] < size) {
+                lvl_id[at] = id[e];
+                lvl_key[at] = key_by_id[id[e]];
+                ++at;
+            }
+        out += total;
+        __syncthreads();  // wsum is read
+    }
 }
 // slot ids from int64 query ids (out-of-range ids become -1) and the sweep sort
 // key: high 32 bits = group (predecessor mode: level and one of kBands id bands
@@ -2471,37 +2538,28 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
     }
     if (e != cudaSuccess) return T->set_err(CT_ERR_NOMEM, "screen prep allocation: %s", cudaGetErrorString(e));
     e = ct::compute_order(T->coords_raw, n, T->d, 1, S->hil_order, st, S->hil_key, S->bounds);
-    std::vector<int> order_h(n);
-    std::vector<unsigned long long> key_h(n);
     if (e == cudaSuccess) {
         iota_kernel<<<grid_for(S->rows_pad), 256, 0, st>>>(S->b_id_ds, S->rows_pad, n);
         split_blocked_kernel<<<152 * 8, 256, 0, st>>>(T->vnat, m, S->b_id_ds, S->rows_pad, S->ds_hi, S->ds_lo);
-        point_scalars_kernel<<<grid_for(n), 256, 0, st>>>(T->vnat, T->p, T->xs, n, m, T->d, S->vn, S->isp, S->xmax);
+        point_scalars_kernel<<<grid_for(n, 64), 64, 0, st>>>(T->vnat, T->p, T->xs, n, m, T->d, S->vn, S->isp, S->xmax);
         e = cudaMemsetAsync(S->isp_max, 0, sizeof(unsigned), st);
         if (e == cudaSuccess) e = cudaMemsetAsync(S->xmax_max, 0, sizeof(unsigned), st);
         if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->isp, n, S->isp_max);
         if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->xmax, n, S->xmax_max);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(order_h.data(), S->hil_order, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(key_h.data(), S->hil_key, 8 * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return T->set_err(CT_ERR_CUDA, "screen prep: %s", cudaGetErrorString(e));
-    // level rows: the Hilbert order filtered to ids < size (stable, so still key-sorted)
-    std::vector<int> lid(S->lvl_rows, -1);
-    std::vector<unsigned long long> lkey(S->lvl_rows, ~0ULL);
     std::vector<long long> meta;
     for (const auto& L : S->levels) {
-        long long r = L.row_off;
-        for (long long i = 0; i < n; ++i) {
-            int id = order_h[i];
-            if (id < L.size) { lid[r] = id; lkey[r] = key_h[id]; ++r; }
-        }
         meta.push_back(L.size); meta.push_back(L.row_off); meta.push_back(L.rows_pad);
     }
-    e = cudaMemcpyAsync(S->lvl_id, lid.data(), sizeof(int) * S->lvl_rows, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(S->lvl_key, lkey.data(), 8 * S->lvl_rows, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(S->lvl_meta, meta.data(), sizeof(long long) * meta.size(), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->lvl_id, 0xff, sizeof(int) * S->lvl_rows, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->lvl_key, 0xff, 8 * S->lvl_rows, st);
+    if (e == cudaSuccess) {
+        build_levels_kernel<<<(unsigned)S->levels.size(), 1024, 0, st>>>(S->hil_order, S->hil_key, n, S->lvl_meta,
+                                                                         S->lvl_id, S->lvl_key);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) {
         split_blocked_kernel<<<152 * 8, 256, 0, st>>>(T->vnat, m, S->lvl_id, S->lvl_rows, S->lvl_hi, S->lvl_lo);
         const float ec = err_coef_for(m);
@@ -2509,9 +2567,9 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
                                                                     S->isp, S->xmax, ec, S->rec_ds);
         build_records_kernel<<<grid_for(S->lvl_rows), 256, 0, st>>>(S->lvl_id, S->lvl_rows, T->xs, T->d, S->vn,
                                                                     S->isp, S->xmax, ec, S->rec_lvl);
-        build_group_records_kernel<<<grid_for(S->rows_pad / (TC / 2)), 256, 0, st>>>(S->b_id_ds, S->rows_pad, T->xs,
+        build_group_records_kernel<<<grid_for(S->rows_pad / (TC / 2) * 32), 256, 0, st>>>(S->b_id_ds, S->rows_pad, T->xs,
                                                                                     T->d, S->vn, S->isp, ec, S->rec_ds);
-        build_group_records_kernel<<<grid_for(S->lvl_rows / (TC / 2)), 256, 0, st>>>(S->lvl_id, S->lvl_rows, T->xs,
+        build_group_records_kernel<<<grid_for(S->lvl_rows / (TC / 2) * 32), 256, 0, st>>>(S->lvl_id, S->lvl_rows, T->xs,
                                                                                      T->d, S->vn, S->isp, ec, S->rec_lvl);
         e = cudaGetLastError();
     }
@@ -3201,7 +3259,7 @@ int ct_tree::knn_screened_points(const float* qv, const float* qp, const float* 
     if (e == cudaSuccess) e = cudaMemcpyAsync(p + n0, qp, sizeof(float) * nq, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) {
         scale_rows_kernel<<<grid_for(nq * d), 256, 0, st>>>(qcoords, nq, d, inv_ls, xs + n0 * d);
-        point_scalars_kernel<<<grid_for(nq), 256, 0, st>>>(vnat + n0 * m, p + n0, xs + n0 * d, nq, m, d,
+        point_scalars_kernel<<<grid_for(nq, 64), 64, 0, st>>>(vnat + n0 * m, p + n0, xs + n0 * d, nq, m, d,
                                                          S->vn + n0, S->isp + n0, S->xmax + n0);
         iota64_kernel<<<grid_for(nq), 256, 0, st>>>(ids, nq, n);
         e = cudaGetLastError();

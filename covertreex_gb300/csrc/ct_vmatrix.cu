@@ -30,28 +30,42 @@
 namespace ct {
 namespace vmat {
 
+// x / b, correctly rounded, from y = the correctly rounded 1 / b: q = x y, then one residual step
+// (Markstein's theorem: three operations where the general division takes about twelve, on a chip
+// with two FP64 operations a clock per SM).  An infinite or NaN quotient is returned as it is.
+__device__ __forceinline__ double div_by(double x, double b, double y) {
+    const double q = x * y;
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return q;
+    return fma(fma(-b, q, x), y, q);
+}
+
+// Kernel value; ls2 = {max(ls, 1e-12), 1 / it} for Matern, {its square, 1 / that} for RBF.
 __device__ __forceinline__ double kernel_f64(const double* __restrict__ x, const double* __restrict__ z, int d,
-                                             int kt, double var, double ls) {
+                                             int kt, double var, double2 ls2) {
     double sq = 0.0;
     for (int c = 0; c < d; ++c) {
         const double t = x[c] - z[c];
         sq += t * t;
     }
-    const double denom = ls > 1e-12 ? ls : 1e-12;
     if (kt == 1) {
-        const double a = sqrt(5.0) * (sqrt(sq) / denom);
-        return var * (1.0 + a + (a * a) / 3.0) * exp(-a);
+        const double a = sqrt(5.0) * div_by(sqrt(sq), ls2.x, ls2.y);
+        return var * (1.0 + a + div_by(a * a, 3.0, 1.0 / 3.0)) * exp(-a);
     }
-    return var * exp(-0.5 * sq / (denom * denom));
+    return var * exp(div_by(-0.5 * sq, ls2.x, ls2.y));
+}
+inline double2 scale_of(int kt, double ls) {
+    const double denom = ls > 1e-12 ? ls : 1e-12;
+    const double b = kt == 1 ? denom : denom * denom;
+    return make_double2(b, 1.0 / b);
 }
 
 // A[i][j] = K(z_i, z_j), plus 1e-6 var on the diagonal (host_backend.py:210-211).
-__global__ void kmm_kernel(const double* __restrict__ z, int m, int d, int kt, double var, double ls,
+__global__ void kmm_kernel(const double* __restrict__ z, int m, int d, int kt, double var, double2 ls2,
                            double* __restrict__ A) {
     const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (e >= (long long)m * m) return;
     const int i = (int)(e / m), j = (int)(e - (long long)i * m);
-    double v = kernel_f64(z + (size_t)i * d, z + (size_t)j * d, d, kt, var, ls);
+    double v = kernel_f64(z + (size_t)i * d, z + (size_t)j * d, d, kt, var, ls2);
     if (i == j) v += 1e-6 * var;
     A[e] = v;
 }
@@ -158,78 +172,109 @@ __global__ void __launch_bounds__(128) trinv_kernel(const double* __restrict__ L
 
 // Kc[r][t] = K(x_{r0+r}, z_t) for r < rows (grid-stride: the grid may be capped).
 __global__ void kxm_kernel(const double* __restrict__ x, long long r0, long long rows, const double* __restrict__ z,
-                           int m, int d, int kt, double var, double ls, double* __restrict__ Kc) {
+                           int m, int d, int kt, double var, double2 ls2, double* __restrict__ Kc) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < rows * m;
          e += (long long)gridDim.x * blockDim.x) {
         const long long r = e / m;
         const int t = (int)(e - r * m);
-        Kc[e] = kernel_f64(x + (size_t)(r0 + r) * d, z + (size_t)t * d, d, kt, var, ls);
+        Kc[e] = kernel_f64(x + (size_t)(r0 + r) * d, z + (size_t)t * d, d, kt, var, ls2);
     }
 }
 
-// Vc[r][j] = sum_{t <= j} Kc[r][t] Li[j][t]; 32 x 32 tiles, 256 threads, 2 x 2 each, a
-// block looping over tiles when the grid is capped.  GB300's FP64 rate is low (one block
-// of eight warps fills an SM's FP64 pipe), so a serving build runs these kernels on a
-// capped grid (ct_set_cta_budget): the other SMs stay free of build blocks, whose shared
-// memory would keep the screened form's large blocks off an SM.
+// Vc[r][j] = sum_{t <= j} Kc[r][t] Li[j][t] in tiles of R x 32, 256 threads, a block looping
+// over tiles when the grid is capped.  GB300's FP64 rate is low (two FMAs a clock per SM: one
+// block of eight warps fills it), so a serving build runs these kernels on a capped grid
+// (ct_set_cta_budget): the other SMs stay free of build blocks, whose shared memory would keep
+// the screened form's large blocks off an SM.
+// R = 32 (2 x 2 outputs per thread) when its tiles fill the chip; R = 8 or 2 for few rows, where a
+// 32-row tile would spend its SM's FP64 pipe on padding (one new point, m = 256: 83 us in 32-row
+// tiles).  Every output is one chain of FMAs in t order whatever the tile, so a row's V does not
+// depend on the rows embedded with it.
 constexpr int GT = 32;
 constexpr int GK = 32;
+template <int R>
 __device__ __forceinline__ void dgemm_lt_tile(const double* __restrict__ Kc, long long rows,
                                               const double* __restrict__ Li, int m, double* __restrict__ Vc,
-                                              double (*As)[GT + 1], double (*Bs)[GT + 1], long long r0, int j0) {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[2][2];
+                                              double (*As)[R + 1], double (*Bs)[GT + 1], long long r0, int j0) {
+    constexpr int U = R == 32 ? 2 : 1;  // outputs per thread on either side
+    const int tx = R == 32 ? threadIdx.x & 15 : threadIdx.x & 31, ty = R == 32 ? threadIdx.x >> 4 : threadIdx.x >> 5;
+    const bool works = R == 32 || ty < R;
+    double acc[U][U];
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int w = 0; w < 2; ++w) acc[u][w] = 0.0;
+        for (int w = 0; w < U; ++w) acc[u][w] = 0.0;
     const int kend = min(m, j0 + GT);  // Li[j][t] = 0 for t > j
+    // the next K step's elements are loaded while this one is summed
+    constexpr int NB = GT * GK / 256, NA = (R * GK + 255) / 256;
+    double na[NA], nb[NB];
+    auto fetch = [&](int t0) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int e = threadIdx.x + 256 * i, j = j0 + e / GK, t = t0 + e % GK;
+            nb[i] = (j < m && t < m) ? Li[(size_t)j * m + t] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int e = threadIdx.x + 256 * i, t = t0 + e % GK;
+            const long long row = r0 + e / GK;
+            na[i] = (e < R * GK && row < rows && t < m) ? Kc[row * m + t] : 0.0;
+        }
+    };
+    fetch(0);
     for (int t0 = 0; t0 < kend; t0 += GK) {
-        for (int e = threadIdx.x; e < GT * GK; e += 256) {
-            const int rr = e / GK, tt = e - rr * GK;
-            const int t = t0 + tt;
-            const long long row = r0 + rr;
-            As[tt][rr] = (row < rows && t < m) ? Kc[row * m + t] : 0.0;
-            const int j = j0 + rr;
-            Bs[tt][rr] = (j < m && t < m) ? Li[(size_t)j * m + t] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int e = threadIdx.x + 256 * i;
+            Bs[e % GK][e / GK] = nb[i];
+        }
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int e = threadIdx.x + 256 * i;
+            if (e < R * GK) As[e % GK][e / GK] = na[i];
         }
         __syncthreads();
+        if (t0 + GK < kend) fetch(t0 + GK);
+        if (works) {
 #pragma unroll 8
-        for (int tt = 0; tt < GK; ++tt) {
-            double a[2], b[2];
+            for (int tt = 0; tt < GK; ++tt) {
+                double a[U], b[U];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                a[u] = As[tt][ty + 16 * u];
-                b[u] = Bs[tt][tx + 16 * u];
+                for (int u = 0; u < U; ++u) {
+                    a[u] = As[tt][ty + 16 * u];
+                    b[u] = Bs[tt][tx + 16 * u];
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int w = 0; w < U; ++w) acc[u][w] = fma(a[u], b[w], acc[u][w]);
             }
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-#pragma unroll
-                for (int w = 0; w < 2; ++w) acc[u][w] = fma(a[u], b[w], acc[u][w]);
         }
         __syncthreads();
     }
+    if (!works) return;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < U; ++u) {
         const long long row = r0 + ty + 16 * u;
         if (row >= rows) continue;
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
+        for (int w = 0; w < U; ++w) {
             const int j = j0 + tx + 16 * w;
             if (j < m) Vc[row * m + j] = acc[u][w];
         }
     }
 }
 
+template <int R>
 __global__ void __launch_bounds__(256) dgemm_lt_kernel(const double* __restrict__ Kc, long long rows,
                                                        const double* __restrict__ Li, int m,
                                                        double* __restrict__ Vc) {
-    __shared__ double As[GK][GT + 1];
+    __shared__ double As[GK][R + 1];
     __shared__ double Bs[GK][GT + 1];
     const int tiles_j = (m + GT - 1) / GT;
-    const long long tiles = tiles_j * ((rows + GT - 1) / GT);
+    const long long tiles = tiles_j * ((rows + R - 1) / R);
     for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x)  // grid-stride: the grid may be capped
-        dgemm_lt_tile(Kc, rows, Li, m, Vc, As, Bs, (tile / tiles_j) * GT, (int)(tile % tiles_j) * GT);
+        dgemm_lt_tile<R>(Kc, rows, Li, m, Vc, As, Bs, (tile / tiles_j) * R, (int)(tile % tiles_j) * GT);
 }
 
 // One warp per row: p = max(var - ||v||^2, 1e-9) in FP64 (fixed summation order),
@@ -264,7 +309,7 @@ cudaError_t vmatrix_factor(const double* z, int m, int d, int kt, double var, do
     const long long mm = (long long)m * m;
     cudaError_t e = cudaMemsetAsync(status_dev, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    kmm_kernel<<<(unsigned)((mm + 255) / 256), 256, 0, st>>>(z, m, d, kt, var, ls, L);
+    kmm_kernel<<<(unsigned)((mm + 255) / 256), 256, 0, st>>>(z, m, d, kt, var, scale_of(kt, ls), L);
     for (int p0 = 0; p0 < m; p0 += CB) {
         const int b = m - p0 < CB ? m - p0 : CB;
         potrf_diag_kernel<<<1, dim3(CB, CB), 0, st>>>(L, m, p0, b, status_dev);
@@ -305,9 +350,12 @@ cudaError_t vmatrix_embed(const double* x, long long n, int d, const double* z, 
     for (long long r0 = 0; r0 < n; r0 += chunk) {
         const long long rows = n - r0 < chunk ? n - r0 : chunk;
         const long long el = rows * m;
-        kxm_kernel<<<capped((el + 255) / 256), 256, 0, st>>>(x, r0, rows, z, m, d, kt, var, ls, kc);
-        const long long tiles = (long long)((m + GT - 1) / GT) * ((rows + GT - 1) / GT);
-        dgemm_lt_kernel<<<capped(tiles), 256, 0, st>>>(kc, rows, Li, m, vc);
+        kxm_kernel<<<capped((el + 255) / 256), 256, 0, st>>>(x, r0, rows, z, m, d, kt, var, scale_of(kt, ls), kc);
+        // the tallest tiles that still give every SM a few blocks
+        const long long tj = (m + GT - 1) / GT;
+        if (tj * ((rows + 31) / 32) >= 304) dgemm_lt_kernel<32><<<capped(tj * ((rows + 31) / 32)), 256, 0, st>>>(kc, rows, Li, m, vc);
+        else if (tj * ((rows + 7) / 8) >= 152) dgemm_lt_kernel<8><<<capped(tj * ((rows + 7) / 8)), 256, 0, st>>>(kc, rows, Li, m, vc);
+        else dgemm_lt_kernel<2><<<capped(tj * ((rows + 1) / 2)), 256, 0, st>>>(kc, rows, Li, m, vc);
         finalize_rows_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>(vc, rows, m, var, V + r0 * m,
                                                                                p + r0);
         nl += 3;
