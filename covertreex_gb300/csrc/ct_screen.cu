@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <functional>
 #include <type_traits>
 #include <tuple>
 #include <vector>
@@ -977,6 +978,10 @@ struct RescoreParams {
     const unsigned* xmax_max;    // bits of the dataset's largest xmax
     const unsigned* isp_max;     // bits of the dataset's largest 1 / sqrt(p)
     const unsigned* qtau;        // per query (slot / parts): the sweep's smallest part threshold (d^2 bits)
+    // rows of the digit pass instead of slots: row -> query (index into qtau), and the rows whose
+    // survivors do not fit (set to 1, left to the exhaustive kernels)
+    const int* row_query;
+    int* row_bad;
 };
 
 // ---------------------------------------------------------- double-float
@@ -1168,25 +1173,38 @@ __device__ __forceinline__ void warp_dots(const float* __restrict__ V, int m, co
     }
 }
 
+// Kernel value of a squared scaled distance, in double-float arithmetic.
+__device__ __forceinline__ df kernel_value_df(const RescoreParams& P, df d2) {
+    if (P.kernel_type == 0) return df_mulf(df_exp(df{-0.5f * d2.h, -0.5f * d2.l}), P.var);
+    const df a = df_mul(df_sqrt(d2), CT_DF(2.23606797749978969641));
+    const df poly = df_add(df_add(df{1.f, 0.f}, a), df_mul(df_mul(a, a), CT_DF(1.0 / 3.0)));
+    return df_mulf(df_mul(poly, df_exp(df_neg(a))), P.var);
+}
+// The same of two points, from their raw coordinates (both loaded before the chain).
+__device__ __forceinline__ df kernel_value_df(const RescoreParams& P, int q, int c) {
+    float x[kMaxD], y[kMaxD];
+#pragma unroll
+    for (int a = 0; a < kMaxD; ++a) {
+        x[a] = a < P.d ? P.coords[(size_t)q * P.d + a] : 0.f;
+        y[a] = a < P.d ? P.coords[(size_t)c * P.d + a] : 0.f;
+    }
+    df d2 = df{0.f, 0.f};
+#pragma unroll
+    for (int a = 0; a < kMaxD; ++a) {
+        if (a >= P.d) break;
+        const df t = df_two_sum(x[a], -y[a]);  // exact
+        const df u = df_mul(t, df{P.inv_ls_df[2 * a], P.inv_ls_df[2 * a + 1]});
+        d2 = df_add(d2, df_mul(u, u));
+    }
+    return kernel_value_df(P, d2);
+}
+
 // Exact residual distance of one pair from its double-float V dot product: the
 // kernel value from the f32 coordinates, the normalisation and the square root, in
 // double-float arithmetic (one lane per pair).
 __device__ __forceinline__ float exact_from_dot(const RescoreParams& P, int q, int c, df dot) {
     if (q == c) return 0.f;
-    df d2 = df{0.f, 0.f};
-    for (int a = 0; a < P.d; ++a) {
-        const df t = df_two_sum(P.coords[(size_t)q * P.d + a], -P.coords[(size_t)c * P.d + a]);  // exact
-        const df u = df_mul(t, df{P.inv_ls_df[2 * a], P.inv_ls_df[2 * a + 1]});
-        d2 = df_add(d2, df_mul(u, u));
-    }
-    df kv;
-    if (P.kernel_type == 0) {
-        kv = df_mulf(df_exp(df{-0.5f * d2.h, -0.5f * d2.l}), P.var);
-    } else {
-        const df a = df_mul(df_sqrt(d2), CT_DF(2.23606797749978969641));
-        const df poly = df_add(df_add(df{1.f, 0.f}, a), df_mul(df_mul(a, a), CT_DF(1.0 / 3.0)));
-        kv = df_mulf(df_mul(poly, df_exp(df_neg(a))), P.var);
-    }
+    const df kv = kernel_value_df(P, q, c);
     const float pq = P.p[q], pc = P.p[c];
     const float ph = __fmul_rn(pq, pc);
     df pp = df_fast(ph, __fmaf_rn(pq, pc, -ph));  // exact product
@@ -1311,7 +1329,10 @@ __global__ void rescore_kernel(RescoreParams P) {
     const int slot = P.order ? P.order[w / P.parts] * P.parts + (int)(w % P.parts) : (int)w;
     const int c0 = P.surv_cnt[2 * slot];
     const int c1 = P.surv_cnt[2 * slot + 1];
-    if (c0 > P.half_cap || c1 > P.half_cap) return;  // handled by the exhaustive pass
+    if (c0 > P.half_cap || c1 > P.half_cap) {  // handled by the exhaustive pass
+        if (P.row_bad && lane == 0) P.row_bad[slot] = 1;
+        return;
+    }
     const int q = P.slot_id[slot];
     if (q < 0) {
         for (int j = lane; j < P.k; j += 32) { P.out_idx[(size_t)slot * P.k + j] = -1; P.out_dist[(size_t)slot * P.k + j] = CT_FLT_MAX; }
@@ -1331,7 +1352,7 @@ __global__ void rescore_kernel(RescoreParams P) {
     // the threshold it ended with: any part's k-th upper bound) are dropped before any row
     // is read; the others are compacted into keys (ids in the low bits)
     int count = 0;
-    const float tq = __uint_as_float(__ldcg(&P.qtau[slot / P.parts]));
+    const float tq = __uint_as_float(__ldcg(&P.qtau[P.row_query ? P.row_query[slot] : slot / P.parts]));
     {
         const float thr = (1.f - tq) * (1.f - 2e-6f) / isq;
         for (int base = 0; base < c0 + c1; base += 32) {
@@ -1344,13 +1365,17 @@ __global__ void rescore_kernel(RescoreParams P) {
                 keep = P.survb[o] >= thr;
             }
             const unsigned mk = __ballot_sync(0xffffffffu, keep);
+            if (count + __popc(mk) > RBUF) {  // (digit rows only: a slot's lists fit)
+                if (lane == 0) P.row_bad[slot] = 1;
+                return;
+            }
             if (keep) keys[count + __popc(mk & ((1u << lane) - 1u))] = (unsigned long long)(unsigned)cid;
             count += __popc(mk);
         }
         __syncwarp();
     }
-    // ---- F: certified FP32 bounds of every remaining survivor
-    for (int base = 0; base < count; base += 32) {
+    // ---- F: certified FP32 bounds of every remaining survivor (a digit row's own bounds are tighter)
+    for (int base = 0; !P.row_bad && base < count; base += 32) {
         const int ci = base + lane;
         const int cid = ci < count ? (int)(unsigned)(keys[ci] & 0xffffffffULL) : -1;
         const int nb = count - base < 32 ? count - base : 32;
@@ -1380,7 +1405,7 @@ __global__ void rescore_kernel(RescoreParams P) {
     // tau: the k-th smallest du2 (bisection over the bit patterns of these non-negative
     // floats), plus the margin of the seeded thresholds; every survivor when fewer than k
     float tau = CT_FLT_MAX;
-    if (count > k) {
+    if (count > k && !P.row_bad) {
         unsigned lo = 0, hi = 0x3f800000u;  // du2 <= 1
         while (lo < hi) {
             const unsigned mid = lo + ((hi - lo) >> 1);
@@ -1401,7 +1426,7 @@ __global__ void rescore_kernel(RescoreParams P) {
     for (int base = 0; base < count; base += 32) {
         const int ci = base + lane;
         unsigned long long key = ci < count ? keys[ci] : 0ULL;
-        const bool keep = ci < count && __uint_as_float((unsigned)(key >> 32)) <= tau;
+        const bool keep = ci < count && __uint_as_float((unsigned)(key >> 32)) <= tau;  // (a digit row's: 0)
         const unsigned mask = __ballot_sync(0xffffffffu, keep);
         __syncwarp();  // every lane has read its key before the ids overwrite du2s
         if (keep) kept[nk + __popc(mask & ((1u << lane) - 1u))] = (int)(unsigned)(key & 0xffffffffULL);
@@ -1541,6 +1566,7 @@ struct State {
     unsigned* isp_max = nullptr;            // bits of max 1/sqrt(p) over the dataset rows
     float *rec_lvl = nullptr, *rec_ds = nullptr;  // sweep candidate records, tile order
     unsigned* xmax_max = nullptr;                 // bits of max |x| over the dataset rows
+    unsigned* vn_max = nullptr;                   // bits of max ||v|| over the dataset rows
     double* inv_ls64 = nullptr;
     float* inv_ls_df = nullptr;             // (hi, lo) float pairs of 1 / lengthscale
     int* status = nullptr;
@@ -2361,7 +2387,8 @@ __global__ void seed_tau_kernel(RescoreParams R, const unsigned long long* __res
 
 __global__ void max_bits_kernel(const float* __restrict__ x, long long n, unsigned* __restrict__ out) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) atomicMax(out, __float_as_uint(fabsf(x[i])));
+    const unsigned m = __reduce_max_sync(0xffffffffu, i < n ? __float_as_uint(fabsf(x[i])) : 0u);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
 // rowmap (A row -> dataset row) and a_slot (A row -> slot) from a sorted slot list
@@ -2438,6 +2465,8 @@ __global__ void merge_parts_kernel(const long long* __restrict__ pidx, const flo
     }
 }
 
+#include "ct_digits.cuh"
+
 static inline unsigned grid_for(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
 static float err_coef_for(int m) {
@@ -2471,6 +2500,195 @@ static cudaError_t launch_sweep(const MMAParams& P, int mode, int ncta, cudaStre
     return cudaGetLastError();
 }
 
+// Host side of the digit pass: queries (index of the call, dataset id), ascending by id, searched over
+// candidates [0, n) or their predecessors, on stream st.  Results land in idx / dist ([nuq][k]);
+// bad[r] = 1 where a row is left to the exhaustive kernels.  All scratch is stream-ordered.
+struct DigitRun {
+    long long *idx = nullptr;
+    float* dist = nullptr;
+    int *qidx = nullptr, *bad = nullptr;
+    long long rows = 0;
+};
+// Estimated microseconds of both exhaustive passes, from calls with 4 .. 1102 such queries over 32768,
+// 131072 and 262144 rows at m = 256 and 512: the kernels below at 1e-7 per pair and column of V for slots
+// that their FP32 filter serves and 5e-7 (a thousand queries) to 1.4e-6 (55) for the others, the digit pass at 4.3e-8 after 200 us and the
+// split of the dataset.  Both sides at the line: 512 queries, n = 131072, m = 256: 1.98 ms against 2.05;
+// 128 queries, n = 262144, m = 512: 3.13 against 2.96; away from it: 16 queries there 1.29 against 2.84,
+// 512 queries 8.67 against 4.94.
+static bool digits_pay(int m, double filtered, double plain, double total, long long rows) {
+    return m * 1e-7 * (filtered + 10.0 * plain) > 200.0 + 1.1e-5 * (double)rows * m + 4.3e-8 * m * total;
+}
+constexpr size_t kDigitSlabBytes = size_t(4) << 30;
+constexpr int kDigitBatch = 4096;      // rows per batch (their survivor lists are 32 KiB each)
+
+static cudaError_t digit_pass(const RescoreParams& R0, const unsigned* vn_max, unsigned* qtau, long long n,
+                              const std::vector<std::pair<int, int>>& uq, int sms, cudaStream_t st, DigitRun* D,
+                              std::vector<int>* bad_h, int* status_h, long long* launches) {
+    const int m = R0.m, k = R0.k, nuq = (int)uq.size();
+    const long long pad = (nuq + TQ - 1) / TQ * TQ, tiles = pad / TQ;
+    const long long cmax = R0.predecessor ? uq.back().second : n;
+    // the dataset's digits in slabs of bounded size (one, but for the largest datasets)
+    const long long slab_max = std::max<long long>(DN, (long long)(kDigitSlabBytes / (sizeof(bf16) * DS * m)) / DN * DN);
+    const long long brows = std::min(slab_max, std::max<long long>(DN, (cmax + DN - 1) / DN * DN));
+    const int nslabs = (int)std::max<long long>(1, (cmax + brows - 1) / brows);
+    const long long batch = std::min<long long>(pad, kDigitBatch), btiles = batch / TQ;
+    std::vector<int> qid(pad, -1), qix(pad, 0);
+    std::vector<long long> cend(tiles, 0);
+    for (int i = 0; i < nuq; ++i) {
+        qix[i] = uq[i].first;
+        qid[i] = uq[i].second;
+        cend[i / TQ] = R0.predecessor ? uq[i].second : n;  // ascending ids: the last of the tile
+    }
+    // Items of the row tiles [g0, g1): a row tile's candidates in chunks of about equal size over the row
+    // tiles, some eight per SM, dealt to the CTAs largest first.
+    struct Plan {
+        std::vector<int4> items;
+        std::vector<int> begin;
+        std::vector<int2> chunks;
+        int total = 0;
+    };
+    auto plan = [&](long long g0, long long g1) {
+        Plan pl;
+        long long sum = 0;
+        for (long long t = g0; t < g1; ++t) sum += std::max<long long>(1, (cend[t] + DN - 1) / DN);
+        struct Sized { long long size; int4 item; };
+        std::vector<Sized> all;
+        for (long long t = g0; t < g1; ++t) {
+            const long long T = std::max<long long>(1, (cend[t] + DN - 1) / DN);
+            const long long want = (T * 8 * sms + sum - 1) / sum;
+            const int nch = (int)std::min<long long>(std::min<long long>(T, kDigitMaxChunks), std::max<long long>(16, want));
+            for (int c = 0; c < nch; ++c) all.push_back({(T + nch - 1 - c) / nch, make_int4((int)(t - g0), c, nch, pl.total)});
+            pl.chunks.push_back(make_int2(nch, pl.total));
+            pl.total += nch;
+        }
+        std::stable_sort(all.begin(), all.end(), [](const Sized& x, const Sized& y) { return x.size > y.size; });
+        const int ctas = (int)std::min<size_t>(sms, all.size());
+        std::vector<std::vector<int4>> of(ctas);
+        std::vector<std::pair<long long, int>> load(ctas);  // a heap: the least loaded CTA first
+        for (int b = 0; b < ctas; ++b) load[b] = {0, b};
+        const auto more = std::greater<std::pair<long long, int>>();
+        for (const Sized& it : all) {
+            std::pop_heap(load.begin(), load.end(), more);
+            load.back().first += it.size;
+            of[load.back().second].push_back(it.item);
+            std::push_heap(load.begin(), load.end(), more);
+        }
+        for (const auto& v : of) {
+            pl.begin.push_back((int)pl.items.size());
+            pl.items.insert(pl.items.end(), v.begin(), v.end());
+        }
+        pl.begin.push_back((int)pl.items.size());
+        return pl;
+    };
+    std::vector<Plan> plans;
+    size_t max_items = 0;
+    for (long long r0 = 0; r0 < pad; r0 += batch) {
+        plans.push_back(plan(r0 / TQ, std::min(pad, r0 + batch) / TQ));
+        max_items = std::max(max_items, plans.back().items.size());
+    }
+    cudaError_t e = cudaSuccess;
+    void* p[16] = {nullptr};
+    int np = 0;
+    auto A = [&](size_t bytes) -> void* {
+        void* q = nullptr;
+        if (e == cudaSuccess) e = cudaMallocAsync(&q, bytes ? bytes : 16, st);
+        if (e == cudaSuccess) p[np++] = q;
+        return q;
+    };
+    DigitParams P{};
+    bf16* a = (bf16*)A(sizeof(bf16) * DS * (size_t)batch * m);
+    bf16* b = (bf16*)A(sizeof(bf16) * DS * (size_t)brows * m);
+    int* qid_d = (int*)A(sizeof(int) * pad);
+    long long* cend_d = (long long*)A(sizeof(long long) * tiles);
+    int4* items_d = (int4*)A(sizeof(int4) * max_items);
+    int* begin_d = (int*)A(sizeof(int) * (sms + 1));
+    int2* chunks_d = (int2*)A(sizeof(int2) * btiles);
+    unsigned* vmax = (unsigned*)A(sizeof(unsigned));
+    float* scale = (float*)A(sizeof(float));
+    P.surv = (int*)A(sizeof(int) * 2 * (size_t)batch * kDigitCap);
+    P.survb = (float*)A(sizeof(float) * 2 * (size_t)batch * kDigitCap);
+    P.cnt = (int*)A(sizeof(int) * 2 * (size_t)batch);
+    P.minima = (float*)A(sizeof(float) * max_items * TQ * 2 * kDigitGroups);
+    P.status = (int*)A(sizeof(int));
+    auto K = [&](void** q, size_t bytes) { if (e == cudaSuccess) e = cudaMallocAsync(q, bytes, st); };
+    K((void**)&D->idx, sizeof(long long) * (size_t)pad * k);
+    K((void**)&D->dist, sizeof(float) * (size_t)pad * k);
+    K((void**)&D->qidx, sizeof(int) * pad);
+    K((void**)&D->bad, sizeof(int) * pad);
+    auto up = [&](void* dst, const void* src, size_t bytes) {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    };
+    up(qid_d, qid.data(), sizeof(int) * pad);
+    up(D->qidx, qix.data(), sizeof(int) * pad);
+    up(cend_d, cend.data(), sizeof(long long) * tiles);
+    if (e == cudaSuccess) e = cudaMemsetAsync(P.status, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(D->bad, 0, sizeof(int) * pad, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(vmax, vn_max, sizeof(unsigned), cudaMemcpyDeviceToDevice, st);
+    const size_t smem = digit_smem().total;
+    const size_t ssmem = (sizeof(unsigned long long) + sizeof(float)) * RBUF * 8;
+    typedef void (*SweepFn)(DigitParams, RescoreParams);
+    static const SweepFn fns[2][2][2] = {  // [pass][kernel type][D > 4]
+        {{digit_sweep_kernel<false, 0, 4>, digit_sweep_kernel<false, 0, 8>}, {digit_sweep_kernel<false, 1, 4>, digit_sweep_kernel<false, 1, 8>}},
+        {{digit_sweep_kernel<true, 0, 4>, digit_sweep_kernel<true, 0, 8>}, {digit_sweep_kernel<true, 1, 4>, digit_sweep_kernel<true, 1, 8>}}};
+    const SweepFn sweep[2] = {fns[0][R0.kernel_type != 0][R0.d > 4], fns[1][R0.kernel_type != 0][R0.d > 4]};
+    for (SweepFn fn : sweep)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem);
+    if (e == cudaSuccess) {
+        gather_max_bits_kernel<<<grid_for(pad), 256, 0, st>>>(R0.vn, qid_d, pad, vmax);
+        digit_scale_kernel<<<1, 1, 0, st>>>(vmax, scale);
+        e = cudaGetLastError();
+        *launches += 2;
+    }
+    for (long long r0 = 0; e == cudaSuccess && r0 < pad; r0 += batch) {
+        const long long rows = std::min(batch, pad - r0);
+        P.a = a; P.b = b;
+        const Plan& pl = plans[r0 / batch];
+        up(items_d, pl.items.data(), sizeof(int4) * pl.items.size());
+        up(begin_d, pl.begin.data(), sizeof(int) * pl.begin.size());
+        up(chunks_d, pl.chunks.data(), sizeof(int2) * pl.chunks.size());
+        P.qid = qid_d + r0; P.qidx = D->qidx + r0; P.items = items_d; P.cta_begin = begin_d; P.tile_chunks = chunks_d;
+        P.cend = cend_d + r0 / TQ; P.scale = scale; P.nz = -0.f;
+        if (e == cudaSuccess) e = cudaMemsetAsync(P.cnt, 0, sizeof(int) * 2 * (size_t)batch, st);
+        if (e != cudaSuccess) break;
+        RescoreParams R = R0;
+        digit_split_kernel<<<152 * 4, 256, 0, st>>>(R.v, m, P.qid, 0, rows, batch, TQ, scale, a);
+        const int grid = (int)pl.begin.size() - 1;
+        // thresholds from every slab, then the survivors of every slab; a single slab's digits are made once
+        for (int ps = 0; ps < 2; ++ps)
+            for (int sl = 0; sl < nslabs; ++sl) {
+                P.base = sl * brows;
+                const long long rows_b = std::min(brows, n - P.base);
+                P.ntiles = (int)((rows_b + DN - 1) / DN);
+                if (nslabs > 1 || (ps == 0 && r0 == 0)) {
+                    digit_split_kernel<<<152 * 16, 256, 0, st>>>(R.v, m, nullptr, P.base, rows_b, brows, DN, scale, b);
+                    ++*launches;
+                }
+                if (ps == 0) {
+                    sweep[0]<<<grid, kDigitThreads, smem, st>>>(P, R);
+                    digit_tau_kernel<<<(unsigned)rows, 256, 0, st>>>(P, R, qtau);
+                } else {
+                    sweep[1]<<<grid, kDigitThreads, smem, st>>>(P, R);
+                }
+                *launches += 2 - ps;
+            }
+        R.slot_id = P.qid; R.nslots = rows; R.order = nullptr; R.parts = 1;
+        R.surv = P.surv; R.survb = P.survb; R.surv_cnt = P.cnt; R.half_cap = kDigitCap;
+        R.row_query = P.qidx; R.row_bad = D->bad + r0;
+        R.out_idx = D->idx + (size_t)r0 * k; R.out_dist = D->dist + (size_t)r0 * k;
+        rescore_kernel<<<(unsigned)((rows + 7) / 8), 256, ssmem, st>>>(R);
+        e = cudaGetLastError();
+        *launches += 2;
+    }
+    D->rows = nuq;
+    bad_h->assign(nuq, 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bad_h->data(), D->bad, sizeof(int) * nuq, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(status_h, P.status, sizeof(int), cudaMemcpyDeviceToHost, st);
+    for (int i = 0; i < np; ++i) cudaFreeAsync(p[i], st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host arrays above, and the rows left over
+    return e;
+}
+
 }  // namespace screen
 }  // namespace ct
 
@@ -2482,7 +2700,7 @@ void ct_tree::release_screen() {
     cudaFree(S->hil_order); cudaFree(S->hil_key); cudaFree(S->ds_hi); cudaFree(S->ds_lo); cudaFree(S->b_id_ds);
     cudaFree(S->lvl_hi); cudaFree(S->lvl_lo); cudaFree(S->lvl_id); cudaFree(S->lvl_key); cudaFree(S->lvl_meta);
     cudaFree(S->vn); cudaFree(S->isp); cudaFree(S->xmax); cudaFree(S->inv_ls64); cudaFree(S->status);
-    cudaFree(S->inv_ls_df); cudaFree(S->isp_max); cudaFree(S->rec_ds); cudaFree(S->rec_lvl); cudaFree(S->xmax_max);
+    cudaFree(S->inv_ls_df); cudaFree(S->isp_max); cudaFree(S->rec_ds); cudaFree(S->rec_lvl); cudaFree(S->xmax_max); cudaFree(S->vn_max);
     cudaFree(S->bounds);
     if (S->slab_done) cudaEventDestroy(S->slab_done);
     delete S;
@@ -2526,6 +2744,7 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
     A((void**)&S->xmax, sizeof(float) * rows_q);
     A((void**)&S->isp_max, sizeof(unsigned));
     A((void**)&S->xmax_max, sizeof(unsigned));
+    A((void**)&S->vn_max, sizeof(unsigned));
     A((void**)&S->rec_ds, sizeof(float) * RT * (S->rows_pad / TC));
     A((void**)&S->rec_lvl, sizeof(float) * RT * (S->lvl_rows / TC));
     A((void**)&S->inv_ls64, sizeof(double) * 64);
@@ -2546,6 +2765,8 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
         if (e == cudaSuccess) e = cudaMemsetAsync(S->xmax_max, 0, sizeof(unsigned), st);
         if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->isp, n, S->isp_max);
         if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->xmax, n, S->xmax_max);
+        if (e == cudaSuccess) e = cudaMemsetAsync(S->vn_max, 0, sizeof(unsigned), st);
+        if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->vn, n, S->vn_max);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     std::vector<long long> meta;
@@ -2911,9 +3132,13 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     unsigned long long* partial = nullptr;
     cudaStream_t aux[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t ev_aux[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    DigitRun digits;
+    int nexh = nfull;  // slots left to the exhaustive kernels
     if (e == cudaSuccess && nfull > 0) {
-        int prio = 0;
-        cudaStreamGetPriority(st, &prio);
+        // above the call's stream: the survivor pass fills the chip with short blocks, and a pass that
+        // started behind it would run after it (vecchia 32768 / 256: 6.57 ms, with priority 5.84)
+        int prio = 0, prio_least = 0;
+        cudaDeviceGetStreamPriorityRange(&prio_least, &prio);
         for (auto& a : aux)
             if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&a, cudaStreamNonBlocking, prio);
         for (auto& v : ev_aux)
@@ -2938,6 +3163,41 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         // fl entries carry bit 31 for slots of the filtered pass until they are grouped
         auto slot_of = [](int v) { return v & 0x7fffffff; };
         auto filt_of = [](int v) { return v < 0 ? 1 : 0; };
+        // The digit pass takes every query with an overflowed slot, over all its candidates; what its
+        // rows cannot hold stays for the kernels below.
+        if (e == cudaSuccess && m <= kDigitMaxM) {
+            std::vector<std::pair<int, int>> uq;  // (dataset id, query of the call)
+            double work[2] = {0, 0}, total = 0;   // pairs of the slots, plain and filtered; of their queries
+            for (int i = 0; i < nfull; ++i) {
+                const int id = sid[slot_of(fl[i])];
+                uq.push_back({id, slot_of(fl[i]) / parts});
+                work[filt_of(fl[i])] += (double)(predecessor ? id : n) / parts;
+            }
+            std::sort(uq.begin(), uq.end());
+            uq.erase(std::unique(uq.begin(), uq.end()), uq.end());
+            for (const auto& x : uq) total += (double)(predecessor ? x.first : n);
+            if (digits_pay(m, work[1], work[0], total, predecessor ? uq.back().first : n)) {
+                for (auto& x : uq) std::swap(x.first, x.second);
+                std::vector<int> bad;
+                int dstatus = 0;
+                e = digit_pass(R, S->vn_max, qtau, n, uq, sms, x0, &digits, &bad, &dstatus, &launches);
+                if (dstatus != 0) status = dstatus;
+                if (e == cudaErrorMemoryAllocation) {  // no room: the kernels below need little
+                    cudaGetLastError();
+                    e = cudaSuccess;
+                    bad.assign(uq.size(), 1);
+                    digits.rows = 0;
+                }
+                std::vector<char> left(nq, 0);
+                for (size_t i = 0; i < uq.size(); ++i) {
+                    if (bad[i]) left[uq[i].first] = 1;
+                    else exh_pairs += predecessor ? (long long)uq[i].second : n;
+                }
+                fl.erase(std::remove_if(fl.begin(), fl.end(), [&](int v) { return !left[slot_of(v) / parts]; }), fl.end());
+                nexh = (int)fl.size();
+            }
+        }
+        if (nexh > 0) {
         std::vector<ExhGroup> groups;
         std::vector<int> gkind;
         auto kind_of = [](int f, int ng) { return f ? (ng > 16 ? 1 : 2) : (ng > 4 ? 0 : 3); };
@@ -2957,19 +3217,19 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
             std::vector<int> tile_of(nq, -1), unit_of(nqt * parts, -1);
             for (long long r = 0; r < nq; ++r) tile_of[sorted_q[r]] = (int)(r / TQ);
             for (size_t u = 0; u < flat_units.size(); ++u) unit_of[flat_units[u].qx] = (int)u;
-            std::vector<std::tuple<int, int, int>> su(nfull);  // (unit, filtered, slot)
-            for (int i = 0; i < nfull; ++i) {
+            std::vector<std::tuple<int, int, int>> su(nexh);  // (unit, filtered, slot)
+            for (int i = 0; i < nexh; ++i) {
                 const int sl = slot_of(fl[i]);
                 const int qi = sl / parts, pp = sl % parts;
                 su[i] = std::make_tuple(unit_of[(long long)tile_of[qi] * parts + pp], filt_of(fl[i]), sl);
             }
             std::sort(su.begin(), su.end());
-            for (int i = 0; i < nfull; ++i) fl[i] = std::get<2>(su[i]);
-            for (int i = 0; i < nfull;) {
+            for (int i = 0; i < nexh; ++i) fl[i] = std::get<2>(su[i]);
+            for (int i = 0; i < nexh;) {
                 const int u = std::get<0>(su[i]), f = std::get<1>(su[i]);
                 const int cap = f ? 32 : XQ;
                 int j = i;
-                while (j < nfull && j - i < cap && std::get<0>(su[j]) == u && std::get<1>(su[j]) == f) ++j;
+                while (j < nexh && j - i < cap && std::get<0>(su[j]) == u && std::get<1>(su[j]) == f) ++j;
                 const int mine = u >= 0 ? flat_units[u].count - flat_units[u].warm : 0;
                 add_group(ExhGroup{i, j - i, u, 0, mine}, kind_of(f, j - i));  // cend: the source's tiles (for chunking)
                 if (u >= 0) exh_pairs += (long long)mine * TC * (j - i);
@@ -2981,17 +3241,17 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
                 if (fa != fb) return fa < fb;
                 return sid[sa] < sid[sb] || (sid[sa] == sid[sb] && sa < sb);
             });
-            for (int i = 0; i < nfull;) {
+            for (int i = 0; i < nexh;) {
                 const int f = filt_of(fl[i]);
                 const int cap = f ? 32 : XQ;
                 int j = i;
-                while (j < nfull && j - i < cap && filt_of(fl[j]) == f) ++j;
+                while (j < nexh && j - i < cap && filt_of(fl[j]) == f) ++j;
                 const long long cend = predecessor ? (long long)sid[slot_of(fl[j - 1])] : n;
                 add_group(ExhGroup{i, j - i, -1, 0, cend}, kind_of(f, j - i));
                 for (int t = i; t < j; ++t) exh_pairs += predecessor ? (long long)sid[slot_of(fl[t])] : n;
                 i = j;
             }
-            for (int i = 0; i < nfull; ++i) fl[i] = slot_of(fl[i]);
+            for (int i = 0; i < nexh; ++i) fl[i] = slot_of(fl[i]);
         }
         // chunking per kind: about target_items CTAs each (warps for the warp items)
         int ktpc[4] = {1, 1, 1, 1}, kchunk[4] = {4096, 4096, 4096, 4096};
@@ -3016,7 +3276,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
                 g.nchunks = (int)((g.cend + kchunk[kd] - 1) / kchunk[kd]);
             }
         }
-        std::vector<int> ibeg(nfull + 1, 0);
+        std::vector<int> ibeg(nexh + 1, 0);
         int rows = 0;
         std::vector<ExhItem> kitems[4];
         for (size_t gi = 0; gi < groups.size(); ++gi) {
@@ -3024,7 +3284,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
             for (int t = g.g0; t < g.g0 + g.ng; ++t) { ibeg[t] = rows; rows += g.nchunks; }
             for (int c = 0; c < g.nchunks; ++c) kitems[gkind[gi]].push_back(ExhItem{(int)gi, c});
         }
-        ibeg[nfull] = rows;
+        ibeg[nexh] = rows;
         // chunk-major within each kind: CTAs in flight read the same candidate rows
         std::vector<ExhItem> xitems;
         int koff[5] = {0, 0, 0, 0, 0};
@@ -3036,7 +3296,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         }
         koff[4] = (int)xitems.size();
         const int nitems = koff[4];
-        AX((void**)&item_begin_d, sizeof(int) * (nfull + 1));
+        AX((void**)&item_begin_d, sizeof(int) * (nexh + 1));
         AX((void**)&partial, sizeof(unsigned long long) * ((size_t)rows * k + 1));
         AX((void**)&groups_d, sizeof(ExhGroup) * (groups.size() + 1));
         AX((void**)&xitems_d, sizeof(ExhItem) * (nitems + 1));
@@ -3044,10 +3304,10 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
             e = cudaMemcpyAsync(groups_d, groups.data(), sizeof(ExhGroup) * groups.size(), cudaMemcpyHostToDevice, x0);
         if (e == cudaSuccess && nitems > 0)
             e = cudaMemcpyAsync(xitems_d, xitems.data(), sizeof(ExhItem) * nitems, cudaMemcpyHostToDevice, x0);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(full_list, fl.data(), sizeof(int) * nfull, cudaMemcpyHostToDevice, x0);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(item_begin_d, ibeg.data(), sizeof(int) * (nfull + 1), cudaMemcpyHostToDevice, x0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(full_list, fl.data(), sizeof(int) * nexh, cudaMemcpyHostToDevice, x0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(item_begin_d, ibeg.data(), sizeof(int) * (nexh + 1), cudaMemcpyHostToDevice, x0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(x0);  // the host vectors may go
-        R.nfull = nfull;
+        R.nfull = nexh;
         const size_t tsmem = tile_smem_bytes(m);
         auto tile_fn = m == 512 ? rescore_tile_kernel<16> : m == 256 ? rescore_tile_kernel<8> : rescore_tile_kernel<0>;
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
@@ -3089,10 +3349,11 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(x0, ev_aux[a], 0);
             }
             if (e == cudaSuccess) {
-                merge_chunks_kernel<<<(unsigned)((nfull + rwpb - 1) / rwpb), 32 * rwpb, rsmem, x0>>>(R, item_begin_d, partial);
+                merge_chunks_kernel<<<(unsigned)((nexh + rwpb - 1) / rwpb), 32 * rwpb, rsmem, x0>>>(R, item_begin_d, partial);
                 e = cudaGetLastError();
                 ++launches;
             }
+        }
         }
         if (e == cudaSuccess) e = cudaEventRecord(ev_aux[4], x0);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_aux[4], 0);
@@ -3111,6 +3372,14 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         e = cudaGetLastError();
         ++launches;
     }
+    if (e == cudaSuccess && digits.rows > 0) {
+        digit_scatter_kernel<<<grid_for(digits.rows * k), 256, 0, st>>>(digits.idx, digits.dist, digits.qidx, digits.bad,
+                                                                        digits.rows, k, (long long*)out_idx, out_dist);
+        e = cudaGetLastError();
+        ++launches;
+    }
+    for (void* q : {(void*)digits.idx, (void*)digits.dist, (void*)digits.qidx, (void*)digits.bad})
+        if (q) cudaFreeAsync(q, st);
     float ms_total = 0.f, ms_a = 0.f, ms_b = 0.f, ms_r = 0.f;
     if (timing && e == cudaSuccess) {
         cudaEventRecord(ev[4], st);
