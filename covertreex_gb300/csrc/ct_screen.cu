@@ -75,6 +75,7 @@ constexpr int GREC = 2;                     // floats per group of 8 candidates
 constexpr int RT = TC * REC + 2 * HBOX + (TC / 8) * GREC;  // floats of one candidate tile's records
 constexpr int kSurvCap = 1024;  // survivors per query slot (two column halves), at most RBUF
 constexpr int RBUF = 1024;                  // rescoring sort buffer (power of two)
+constexpr int RSMALL = 512;                 // of the survivor pass's first kernel
 // Overflowed query slots with |v_q| / sqrt(p_q) up to this go to the filtered exhaustive
 // pass (certified FP32 bounds first); above it the bounds exclude almost nothing.
 constexpr float kFilterIsq = 256.f;
@@ -941,9 +942,9 @@ __device__ void warp_bitonic_sort(unsigned long long* keys, int len = RBUF) {
     }
 }
 
-__device__ __forceinline__ int sort_len(int fill) {
+__device__ __forceinline__ int sort_len(int fill, int buf = RBUF) {
     int len = 32;
-    while (len < fill && len < RBUF) len <<= 1;
+    while (len < fill && len < buf) len <<= 1;
     return len;
 }
 
@@ -982,6 +983,9 @@ struct RescoreParams {
     // survivors do not fit (set to 1, left to the exhaustive kernels)
     const int* row_query;
     int* row_bad;
+    // survivor pass: slots with more survivors than the first kernel's buffer (filled by it), count
+    int* big_list;
+    int* big_cnt;
 };
 
 // ---------------------------------------------------------- double-float
@@ -1075,12 +1079,13 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& comp, float a, floa
 }
 
 // Load the query slice: lane l holds elements [l*m/32, (l+1)*m/32).
-__device__ __forceinline__ void load_query_slice(const float* row, int m, float (&vq)[32]) {
+template <int PER>
+__device__ __forceinline__ void load_query_slice(const float* row, int m, float (&vq)[PER]) {
     const int lane = threadIdx.x & 31;
     const int per = m >> 5;
     const float* r = row + (size_t)lane * per;
 #pragma unroll
-    for (int t = 0; t < 32; ++t) vq[t] = t < per ? r[t] : 0.f;
+    for (int t = 0; t < PER; ++t) vq[t] = t < per ? r[t] : 0.f;
 }
 
 // One step of the warp reduction of (sum, compensation) pairs: TwoSum of the sums, the
@@ -1117,12 +1122,16 @@ __device__ __forceinline__ void df_combine2(float2& hi, float2& lo, float2 oh, f
     lo = __fadd2_rn(__fadd2_rn(lo, ol), err);
 }
 
-// Dots of the query slice with NC candidate rows at once (independent loads in flight).
-// Lane L sums elements [L m/32, (L+1) m/32) in order; the lanes' pairs are combined by a
-// butterfly over lane offsets 16, 8, 4, 2, 1.
-template <int NC>
-__device__ __forceinline__ void warp_dots(const float* __restrict__ V, int m, const int (&cid)[NC],
-                                          const float (&vq)[32], df (&out)[NC]) {
+// Dots of the query slice with four candidate rows at once (independent loads in flight); lane L returns
+// that of candidate L & 3.  Lane L sums elements [L m/32, (L+1) m/32) in order; the lanes' pairs are
+// combined over lane offsets 16, 8, 4, 2, 1.  Every pair of lanes would get the same value from a step (see
+// df_combine), so the first two steps exchange candidates instead: a lane keeps two of four, then one of
+// two, and 5 steps of 12 shuffles replace 20 of 40 (survivor pass
+// at n = 262144, m = 512: 18.2 -> 15.5 ms).
+template <int PER>
+__device__ __forceinline__ df warp_dots4(const float* __restrict__ V, int m, const int (&cid)[4],
+                                         const float (&vq)[PER]) {
+    constexpr int NC = 4;
     const int lane = threadIdx.x & 31;
     const int per = m >> 5;
     float s[NC], comp[NC];
@@ -1130,7 +1139,7 @@ __device__ __forceinline__ void warp_dots(const float* __restrict__ V, int m, co
     for (int c = 0; c < NC; ++c) { s[c] = 0.f; comp[c] = 0.f; }
     if ((per & 3) == 0) {
 #pragma unroll
-        for (int t4 = 0; t4 < 8; ++t4) {
+        for (int t4 = 0; t4 < PER / 4; ++t4) {
             if (t4 * 4 < per) {
                 float4 x[NC];
 #pragma unroll
@@ -1148,7 +1157,7 @@ __device__ __forceinline__ void warp_dots(const float* __restrict__ V, int m, co
         }
     } else {
 #pragma unroll
-        for (int t = 0; t < 32; ++t) {
+        for (int t = 0; t < PER; ++t) {
             if (t < per) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -1158,19 +1167,30 @@ __device__ __forceinline__ void warp_dots(const float* __restrict__ V, int m, co
             }
         }
     }
-    // Warp reduction in double-float: a butterfly of TwoSum on the (sum, compensation)
-    // pairs, so every lane ends with the same double-float value.
+    const bool hi16 = lane & 16, hi8 = lane & 8;  // keeps candidates 2, 3 / the second of its two
+    float h[2], l[2];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        float hi = s[c], lo = comp[c];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float oh = __shfl_xor_sync(0xffffffffu, hi, off);
-            const float ol = __shfl_xor_sync(0xffffffffu, lo, off);
-            df_combine(hi, lo, oh, ol);
-        }
-        out[c] = df_fast(hi, lo);
+    for (int c = 0; c < 2; ++c) {
+        h[c] = hi16 ? s[c + 2] : s[c];
+        l[c] = hi16 ? comp[c + 2] : comp[c];
+        const float oh = __shfl_xor_sync(0xffffffffu, hi16 ? s[c] : s[c + 2], 16);
+        const float ol = __shfl_xor_sync(0xffffffffu, hi16 ? comp[c] : comp[c + 2], 16);
+        df_combine(h[c], l[c], oh, ol);
     }
+    float hi = hi8 ? h[1] : h[0], lo = hi8 ? l[1] : l[0];
+    {
+        const float oh = __shfl_xor_sync(0xffffffffu, hi8 ? h[0] : h[1], 8);
+        const float ol = __shfl_xor_sync(0xffffffffu, hi8 ? l[0] : l[1], 8);
+        df_combine(hi, lo, oh, ol);
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
+        const float oh = __shfl_xor_sync(0xffffffffu, hi, off);
+        const float ol = __shfl_xor_sync(0xffffffffu, lo, off);
+        df_combine(hi, lo, oh, ol);
+    }
+    const df r = df_fast(hi, lo);  // of candidate lane / 8
+    return df{__shfl_sync(0xffffffffu, r.h, (lane & 3) * 8), __shfl_sync(0xffffffffu, r.l, (lane & 3) * 8)};
 }
 
 // Kernel value of a squared scaled distance, in double-float arithmetic.
@@ -1220,15 +1240,17 @@ __device__ __forceinline__ float exact_from_dot(const RescoreParams& P, int q, i
 }
 #undef CT_DF
 
+template <int BUF = RBUF>
 __device__ __forceinline__ void warp_topk_append(unsigned long long* keys, int& fill, int k, bool has,
                                                  unsigned long long key);
 
 // Plain FP32 dots of the query slice with NC candidate rows (the split of warp_dots,
 // one FMA per element, then a butterfly sum).  Each lane's chain has m/32 roundings
 // and the butterfly 5 more, so |error| <= (m/32 + 7) 2^-24 |v_q| |v_c|.
-template <int NC>
-__device__ __forceinline__ void warp_dots_f32(const float* __restrict__ V, int m, const int (&cid)[NC],
-                                              const float (&vq)[32], float (&out)[NC]) {
+template <int PER>
+__device__ __forceinline__ float warp_dots4_f32(const float* __restrict__ V, int m, const int (&cid)[4],
+                                                const float (&vq)[PER]) {
+    constexpr int NC = 4;
     const int lane = threadIdx.x & 31;
     const int per = m >> 5;
     float s[NC];
@@ -1236,7 +1258,7 @@ __device__ __forceinline__ void warp_dots_f32(const float* __restrict__ V, int m
     for (int c = 0; c < NC; ++c) s[c] = 0.f;
     if ((per & 3) == 0) {
 #pragma unroll
-        for (int t4 = 0; t4 < 8; ++t4) {
+        for (int t4 = 0; t4 < PER / 4; ++t4) {
             if (t4 * 4 < per) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -1251,7 +1273,7 @@ __device__ __forceinline__ void warp_dots_f32(const float* __restrict__ V, int m
         }
     } else {
 #pragma unroll
-        for (int t = 0; t < 32; ++t) {
+        for (int t = 0; t < PER; ++t) {
             if (t < per) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -1261,12 +1283,15 @@ __device__ __forceinline__ void warp_dots_f32(const float* __restrict__ V, int m
             }
         }
     }
+    const bool hi16 = lane & 16, hi8 = lane & 8;  // as in warp_dots4
+    float h[2];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
+    for (int c = 0; c < 2; ++c)
+        h[c] = __fadd_rn(hi16 ? s[c + 2] : s[c], __shfl_xor_sync(0xffffffffu, hi16 ? s[c] : s[c + 2], 16));
+    float r = __fadd_rn(hi8 ? h[1] : h[0], __shfl_xor_sync(0xffffffffu, hi8 ? h[0] : h[1], 8));
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s[c] = __fadd_rn(s[c], __shfl_xor_sync(0xffffffffu, s[c], off));
-        out[c] = s[c];
-    }
+    for (int off = 4; off > 0; off >>= 1) r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, off));
+    return __shfl_sync(0xffffffffu, r, (lane & 3) * 8);
 }
 
 // Certified bounds [dl2, du2] of d^2 = 1 - |rho| for one pair from an FP32 dot with
@@ -1314,32 +1339,41 @@ __device__ __forceinline__ void pair_bounds_f32(const RescoreParams& P, int q, i
 //     by the double-float error of the exact distances, bounds the k-th distance.
 //  E: only survivors with dl2 <= tau are rescored exactly (compensated FP32 dot,
 //     double-float distance); the others cannot enter the top k.
+// One slot's work is a chain of short gathers, so the pass is bound by the warps in flight: a first kernel
+// with buffers of RSMALL survivors and a slice of m / 32 registers (24 warps per SM for m <= 512, not 16)
+// lists the few slots that need more for a second one.  n = 32768, m = 256: 1.72 ms -> 0.90 and 0.3;
+// n = 262144, m = 512: 15.5 -> 13.6 ms.
 // Streaming top-k of E through a sorted shared buffer: entries [0, k) hold the current
 // best, new candidates fill the rest, and a full buffer is re-sorted.  Shared memory per
-// warp: RBUF keys, then RBUF floats (du2, reused for the kept ids).
-__global__ void rescore_kernel(RescoreParams P) {
+// warp: BUF keys, then BUF floats (du2, reused for the kept ids).
+template <int PER, int BUF>
+__global__ void __launch_bounds__(256, PER <= 16 && BUF < RBUF ? 3 : 2) rescore_kernel(RescoreParams P) {
     extern __shared__ unsigned long long rkeys_all[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wpb = blockDim.x / 32;
-    unsigned long long* keys = rkeys_all + (size_t)warp * RBUF;
-    float* du2s = (float*)(rkeys_all + (size_t)wpb * RBUF) + (size_t)warp * RBUF;
+    unsigned long long* keys = rkeys_all + (size_t)warp * BUF;
+    float* du2s = (float*)(rkeys_all + (size_t)wpb * BUF) + (size_t)warp * BUF;
     int* kept = (int*)du2s;
-    const long long w = (long long)blockIdx.x * wpb + warp;
-    if (w >= P.nslots) return;
-    const int slot = P.order ? P.order[w / P.parts] * P.parts + (int)(w % P.parts) : (int)w;
+    // second kernel of the survivor pass: the listed slots; else all (one per warp)
+    const bool listed = BUF == RBUF && P.big_list;
+    const long long nw = listed ? *P.big_cnt : P.nslots;
+    for (long long w = (long long)blockIdx.x * wpb + warp; w < nw; w += (long long)gridDim.x * wpb) {
+    const int slot = listed    ? P.big_list[w]
+                     : P.order ? P.order[w / P.parts] * P.parts + (int)(w % P.parts)
+                               : (int)w;
     const int c0 = P.surv_cnt[2 * slot];
     const int c1 = P.surv_cnt[2 * slot + 1];
     if (c0 > P.half_cap || c1 > P.half_cap) {  // handled by the exhaustive pass
         if (P.row_bad && lane == 0) P.row_bad[slot] = 1;
-        return;
+        continue;
     }
     const int q = P.slot_id[slot];
     if (q < 0) {
         for (int j = lane; j < P.k; j += 32) { P.out_idx[(size_t)slot * P.k + j] = -1; P.out_dist[(size_t)slot * P.k + j] = CT_FLT_MAX; }
-        return;
+        continue;
     }
     const int k = P.k;
-    float vql[32];
+    float vql[PER];
     load_query_slice(P.v + (size_t)q * P.m, P.m, vql);
     // per-query constants of the bounds
     const float isq = P.isp[q];
@@ -1352,6 +1386,7 @@ __global__ void rescore_kernel(RescoreParams P) {
     // the threshold it ended with: any part's k-th upper bound) are dropped before any row
     // is read; the others are compacted into keys (ids in the low bits)
     int count = 0;
+    bool fits = true;
     const float tq = __uint_as_float(__ldcg(&P.qtau[P.row_query ? P.row_query[slot] : slot / P.parts]));
     {
         const float thr = (1.f - tq) * (1.f - 2e-6f) / isq;
@@ -1365,15 +1400,20 @@ __global__ void rescore_kernel(RescoreParams P) {
                 keep = P.survb[o] >= thr;
             }
             const unsigned mk = __ballot_sync(0xffffffffu, keep);
-            if (count + __popc(mk) > RBUF) {  // (digit rows only: a slot's lists fit)
-                if (lane == 0) P.row_bad[slot] = 1;
-                return;
+            if (count + __popc(mk) > BUF) {  // (only digit rows exceed RBUF)
+                if (lane == 0) {
+                    if (BUF == RBUF) P.row_bad[slot] = 1;
+                    else P.big_list[atomicAdd(P.big_cnt, 1)] = slot;
+                }
+                fits = false;
+                break;
             }
             if (keep) keys[count + __popc(mk & ((1u << lane) - 1u))] = (unsigned long long)(unsigned)cid;
             count += __popc(mk);
         }
         __syncwarp();
     }
+    if (!fits) continue;
     // ---- F: certified FP32 bounds of every remaining survivor (a digit row's own bounds are tighter)
     for (int base = 0; !P.row_bad && base < count; base += 32) {
         const int ci = base + lane;
@@ -1382,16 +1422,13 @@ __global__ void rescore_kernel(RescoreParams P) {
         float mydot = 0.f;
         for (int t = 0; t < nb; t += 4) {
             int cc[4];
-            float dots[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int src = __shfl_sync(0xffffffffu, cid, (t + u) & 31);
                 cc[u] = (t + u) < nb ? src : -1;
             }
-            warp_dots_f32<4>(P.v, P.m, cc, vql, dots);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (lane == t + u) mydot = dots[u];
+            const float dot4 = warp_dots4_f32(P.v, P.m, cc, vql);
+            if (lane >> 2 == t >> 2) mydot = dot4;
         }
         if (ci < count) {
             float dl2 = 0.f, du2 = 0.f;  // the query itself: d = 0
@@ -1432,7 +1469,7 @@ __global__ void rescore_kernel(RescoreParams P) {
         if (keep) kept[nk + __popc(mask & ((1u << lane) - 1u))] = (int)(unsigned)(key & 0xffffffffULL);
         nk += __popc(mask);
     }
-    for (int i = lane; i < RBUF; i += 32) keys[i] = ~0ULL;
+    for (int i = lane; i < BUF; i += 32) keys[i] = ~0ULL;
     __syncwarp();
     // ---- E: exact rescoring of the kept survivors
     int fill = k;  // next free position in the buffer
@@ -1443,21 +1480,18 @@ __global__ void rescore_kernel(RescoreParams P) {
         const int nb = nk - base < 32 ? nk - base : 32;
         for (int t = 0; t < nb; t += 4) {
             int cc[4];
-            df dots[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int src = __shfl_sync(0xffffffffu, cid, (t + u) & 31);
                 cc[u] = (t + u) < nb ? src : -1;
             }
-            warp_dots<4>(P.v, P.m, cc, vql, dots);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (lane == t + u) mydot = dots[u];
+            const df dot4 = warp_dots4(P.v, P.m, cc, vql);
+            if (lane >> 2 == t >> 2) mydot = dot4;
         }
         const float mydist = ci < nk ? exact_from_dot(P, q, cid, mydot) : 0.f;
-        warp_topk_append(keys, fill, k, ci < nk, pack_key(mydist, cid));
+        warp_topk_append<BUF>(keys, fill, k, ci < nk, pack_key(mydist, cid));
     }
-    warp_bitonic_sort(keys, sort_len(fill));
+    warp_bitonic_sort(keys, sort_len(fill, BUF));
     for (int j = lane; j < k; j += 32) {
         unsigned long long key = keys[j];
         bool ok = key != ~0ULL;
@@ -1465,17 +1499,20 @@ __global__ void rescore_kernel(RescoreParams P) {
         P.out_dist[(size_t)slot * k + j] = ok ? __uint_as_float((unsigned)(key >> 32)) : CT_FLT_MAX;
     }
     if (lane == 0 && P.evals) atomicAdd((unsigned long long*)P.evals, (unsigned long long)nk);
+    __syncwarp();  // the buffers serve the warp's next slot
+    }
 }
 
+template <int BUF>
 __device__ __forceinline__ void warp_topk_append(unsigned long long* keys, int& fill, int k, bool has,
                                                  unsigned long long key) {
     const int lane = threadIdx.x & 31;
     unsigned mask = __ballot_sync(0xffffffffu, has);
     int added = __popc(mask);
-    if (fill + added > RBUF) {
+    if (fill + added > BUF) {
         __syncwarp();
-        warp_bitonic_sort(keys);
-        for (int i = k + lane; i < RBUF; i += 32) keys[i] = ~0ULL;
+        warp_bitonic_sort(keys, BUF);
+        for (int i = k + lane; i < BUF; i += 32) keys[i] = ~0ULL;
         __syncwarp();
         fill = k;
     }
@@ -1928,16 +1965,13 @@ __global__ void __launch_bounds__(256) rescore_warp_kernel(RescoreParams P, cons
             for (int t = 0; t < 32; t += 4) {
                 if (((hm >> t) & 15u) == 0u) continue;
                 int cc[4];
-                df dd4[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int src = __shfl_sync(0xffffffffu, cid, t + u);
                     cc[u] = (hm >> (t + u)) & 1u ? src : -1;
                 }
-                warp_dots<4>(P.v, m, cc, vql, dd4);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (lane == t + u) mydot = dd4[u];
+                const df dot4 = warp_dots4(P.v, m, cc, vql);
+                if (lane >> 2 == t >> 2) mydot = dot4;
             }
             const float dist = has ? exact_from_dot(P, q, cid, mydot) : 0.f;
             evals += __popc(hm);
@@ -2198,16 +2232,13 @@ __global__ void __launch_bounds__(256, 1) filter_tile_kernel(RescoreParams P, co
                 df mydot = df{0.f, 0.f};
                 for (int t = 0; t < nb; t += 4) {
                     int cc[4];
-                    df dd4[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const int src = __shfl_sync(0xffffffffu, cid, (t + u) & 31);
                         cc[u] = (t + u) < nb ? src : -1;
                     }
-                    warp_dots<4>(P.v, m, cc, vql, dd4);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (lane == t + u) mydot = dd4[u];
+                    const df dot4 = warp_dots4(P.v, m, cc, vql);
+                    if (lane >> 2 == t >> 2) mydot = dot4;
                 }
                 const float dist = has ? exact_from_dot(P, q, cid, mydot) : 0.f;
                 evals += nb;
@@ -2356,13 +2387,10 @@ __global__ void seed_tau_kernel(RescoreParams R, const unsigned long long* __res
         df mydot = df{0.f, 0.f};
         for (int t = 0; t < 32; t += 4) {
             int cc[4];
-            df dots[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) cc[u] = __shfl_sync(0xffffffffu, cid, t + u);
-            warp_dots<4>(R.v, R.m, cc, vql, dots);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (lane == t + u) mydot = dots[u];
+            const df dot4 = warp_dots4(R.v, R.m, cc, vql);
+            if (lane >> 2 == t >> 2) mydot = dot4;
         }
         dist[r] = cid >= 0 ? exact_from_dot(R, q, cid, mydot) : __int_as_float(0x7f800000);
     }
@@ -2466,6 +2494,16 @@ __global__ void merge_parts_kernel(const long long* __restrict__ pidx, const flo
 }
 
 #include "ct_digits.cuh"
+
+typedef void (*RescoreFn)(RescoreParams);
+// The survivor pass for m, with the small buffer or the full one; a slice is m / 32 floats.
+static RescoreFn rescore_fn(int m, bool small) {
+    const int per = m / 32;
+    if (per <= 8) return small ? rescore_kernel<8, RSMALL> : rescore_kernel<8, RBUF>;
+    if (per <= 16) return small ? rescore_kernel<16, RSMALL> : rescore_kernel<16, RBUF>;
+    return small ? rescore_kernel<32, RSMALL> : rescore_kernel<32, RBUF>;
+}
+constexpr size_t rescore_smem(int buf) { return (sizeof(unsigned long long) + sizeof(float)) * buf * 8; }
 
 static inline unsigned grid_for(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
@@ -2625,7 +2663,7 @@ static cudaError_t digit_pass(const RescoreParams& R0, const unsigned* vn_max, u
     if (e == cudaSuccess) e = cudaMemsetAsync(D->bad, 0, sizeof(int) * pad, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(vmax, vn_max, sizeof(unsigned), cudaMemcpyDeviceToDevice, st);
     const size_t smem = digit_smem().total;
-    const size_t ssmem = (sizeof(unsigned long long) + sizeof(float)) * RBUF * 8;
+    const RescoreFn finish = rescore_fn(m, false);
     typedef void (*SweepFn)(DigitParams, RescoreParams);
     static const SweepFn fns[2][2][2] = {  // [pass][kernel type][D > 4]
         {{digit_sweep_kernel<false, 0, 4>, digit_sweep_kernel<false, 0, 8>}, {digit_sweep_kernel<false, 1, 4>, digit_sweep_kernel<false, 1, 8>}},
@@ -2633,7 +2671,7 @@ static cudaError_t digit_pass(const RescoreParams& R0, const unsigned* vn_max, u
     const SweepFn sweep[2] = {fns[0][R0.kernel_type != 0][R0.d > 4], fns[1][R0.kernel_type != 0][R0.d > 4]};
     for (SweepFn fn : sweep)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rescore_smem(RBUF));
     if (e == cudaSuccess) {
         gather_max_bits_kernel<<<grid_for(pad), 256, 0, st>>>(R0.vn, qid_d, pad, vmax);
         digit_scale_kernel<<<1, 1, 0, st>>>(vmax, scale);
@@ -2676,7 +2714,8 @@ static cudaError_t digit_pass(const RescoreParams& R0, const unsigned* vn_max, u
         R.surv = P.surv; R.survb = P.survb; R.surv_cnt = P.cnt; R.half_cap = kDigitCap;
         R.row_query = P.qidx; R.row_bad = D->bad + r0;
         R.out_idx = D->idx + (size_t)r0 * k; R.out_dist = D->dist + (size_t)r0 * k;
-        rescore_kernel<<<(unsigned)((rows + 7) / 8), 256, ssmem, st>>>(R);
+        R.big_list = nullptr;
+        finish<<<(unsigned)((rows + 7) / 8), 256, rescore_smem(RBUF), st>>>(R);
         e = cudaGetLastError();
         *launches += 2;
     }
@@ -2840,7 +2879,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     int *a_slot_x = nullptr, *rowmap_x = nullptr, *slot_id_x = nullptr;  // part-expanded (parts > 1)
     bf16 *al_hi = nullptr, *al_lo = nullptr;
     float* survb = nullptr;
-    int *surv = nullptr, *surv_cnt = nullptr, *full_list = nullptr, *nfull_d = nullptr, *unit_counter = nullptr;
+    int *surv = nullptr, *surv_cnt = nullptr, *full_list = nullptr, *nfull_d = nullptr, *big_list = nullptr, *unit_counter = nullptr;
     int2* unit_jobs_d = nullptr;
     long long* part_idx = nullptr;
     float* part_dist = nullptr;
@@ -2856,7 +2895,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     A((void**)&hist, sizeof(unsigned) * 256 * (size_t)nbh);
     A((void**)&a_slot_lvl, sizeof(int) * rows_q);
     A((void**)&rowmap_lvl, sizeof(int) * rows_q);
-    A((void**)&nfull_d, sizeof(int));
+    A((void**)&nfull_d, 2 * sizeof(int));  // overflowed slots; slots of the survivor pass's second kernel
     A((void**)&evals_d, sizeof(long long));
     A((void**)&qtau, sizeof(unsigned) * nq);
     if (e != cudaSuccess) return set_err(CT_ERR_NOMEM, "screened form allocation: %s", cudaGetErrorString(e));
@@ -3043,6 +3082,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     A((void**)&survb, sizeof(float) * nslots * 2 * (size_t)half_cap);
     A((void**)&surv_cnt, sizeof(int) * 2 * nslots);
     A((void**)&full_list, sizeof(int) * nslots);
+    A((void**)&big_list, sizeof(int) * nslots);
     A((void**)&jobs, sizeof(Job) * (njobs + 1));
     A((void**)&units_d, sizeof(JobUnit) * (flat_units.size() + 1));
     A((void**)&unit_jobs_d, sizeof(int2) * (unit_jobs_h.size() + 1));
@@ -3062,7 +3102,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         e = cudaMemcpyAsync(unit_jobs_d, unit_jobs_h.data(), sizeof(int2) * unit_jobs_h.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(unit_counter, 0, sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(surv_cnt, 0, sizeof(int) * 2 * nslots, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(nfull_d, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(nfull_d, 0, 2 * sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(evals_d, 0, sizeof(long long), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(S->status, 0, sizeof(int), st);
     // ---- sweep
@@ -3103,8 +3143,10 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const size_t fsmem8 = filter_smem_bytes(m, 8), fsmem4 = filter_smem_bytes(m, 4);
     const bool can_filter = m <= 1024 && fsmem8 <= (size_t)smem_optin;
-    const size_t ssmem = (sizeof(unsigned long long) + sizeof(float)) * RBUF * rwpb;  // survivor pass
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem);
+    const RescoreFn surv_fn = rescore_fn(m, true), big_fn = rescore_fn(m, false);  // survivor pass
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(surv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rescore_smem(RSMALL));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(big_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rescore_smem(RBUF));
+    R.big_list = big_list; R.big_cnt = nfull_d + 1;
     // The overflow list first: the exhaustive pass is planned on the host and runs on side
     // streams while the survivor pass runs on the call's stream.
     int nfull = 0, status = 0;
@@ -3121,9 +3163,11 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_ovf, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventRecord(ev_ovf, st);
     if (e == cudaSuccess) {
-        rescore_kernel<<<(unsigned)((nslots + rwpb - 1) / rwpb), 32 * rwpb, ssmem, st>>>(R);
+        const unsigned sblocks = (unsigned)((nslots + rwpb - 1) / rwpb);
+        surv_fn<<<sblocks, 32 * rwpb, rescore_smem(RSMALL), st>>>(R);
+        big_fn<<<std::min(sblocks, 2u * sms), 32 * rwpb, rescore_smem(RBUF), st>>>(R);
         e = cudaGetLastError();
-        ++launches;
+        launches += 2;
     }
     if (e == cudaSuccess) e = cudaEventSynchronize(ev_ovf);
     ExhGroup* groups_d = nullptr;
@@ -3402,7 +3446,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     cudaFreeAsync(a_slot_lvl, st); cudaFreeAsync(rowmap_lvl, st);
     cudaFreeAsync(al_hi, st); cudaFreeAsync(al_lo, st);
     cudaFreeAsync(surv, st); cudaFreeAsync(surv_cnt, st); cudaFreeAsync(survb, st);
-    cudaFreeAsync(full_list, st); cudaFreeAsync(nfull_d, st); cudaFreeAsync(evals_d, st);
+    cudaFreeAsync(full_list, st); cudaFreeAsync(nfull_d, st); cudaFreeAsync(big_list, st); cudaFreeAsync(evals_d, st);
     cudaFreeAsync(jobs, st); cudaFreeAsync(unit_jobs_d, st); cudaFreeAsync(unit_counter, st); cudaFreeAsync(qtau, st);
     if (units_d) cudaFreeAsync(units_d, st);
     if (a_slot_x) cudaFreeAsync(a_slot_x, st);
