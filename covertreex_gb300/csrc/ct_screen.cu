@@ -2547,14 +2547,16 @@ struct DigitRun {
     int *qidx = nullptr, *bad = nullptr;
     long long rows = 0;
 };
-// Estimated microseconds of both exhaustive passes, from calls with 4 .. 1102 such queries over 32768,
-// 131072 and 262144 rows at m = 256 and 512: the kernels below at 1e-7 per pair and column of V for slots
-// that their FP32 filter serves and 5e-7 (a thousand queries) to 1.4e-6 (55) for the others, the digit pass at 4.3e-8 after 200 us and the
-// split of the dataset.  Both sides at the line: 512 queries, n = 131072, m = 256: 1.98 ms against 2.05;
-// 128 queries, n = 262144, m = 512: 3.13 against 2.96; away from it: 16 queries there 1.29 against 2.84,
-// 512 queries 8.67 against 4.94.
-static bool digits_pay(int m, double filtered, double plain, double total, long long rows) {
-    return m * 1e-7 * (filtered + 10.0 * plain) > 200.0 + 1.1e-5 * (double)rows * m + 4.3e-8 * m * total;
+// Estimated microseconds of both exhaustive passes for nslots overflowed slots: the general kernels at
+// 3e-7 per pair and column of V for slots that their FP32 filter serves and 6e-7 for the others, after a
+// latency that grows with the slots; the digit pass at 4.3e-8 after 200 us and the split of the dataset.
+// Both sides, general against digits (m = 256 unless given).  Points against n = 131072: 1024 of them, 53
+// slots overflowed, 1.77 ms against 2.07; 512, 2708 slots, 2.16 against 2.30; 4096, 154 slots, 4.32 against
+// 3.91; 2048 (RBF), 16157 slots, 28.3 against 5.3.  Rows: 500 of n = 65536 at m = 512 (RBF) 11.6 against
+// 2.4; 3000 at m = 128, 155 slots, 1.93 against 1.72; every row of 20000 at m = 96 (RBF) 39.9 against 7.9.
+static bool digits_pay(int m, int nslots, double filtered, double plain, double total, long long rows) {
+    return std::min(300.0, 3.0 * nslots) + m * (3e-7 * filtered + 6e-7 * plain) >
+           200.0 + 1.1e-5 * (double)rows * m + 4.3e-8 * m * total;
 }
 constexpr size_t kDigitSlabBytes = size_t(4) << 30;
 constexpr int kDigitBatch = 4096;      // rows per batch (their survivor lists are 32 KiB each)
@@ -3220,7 +3222,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
             std::sort(uq.begin(), uq.end());
             uq.erase(std::unique(uq.begin(), uq.end()), uq.end());
             for (const auto& x : uq) total += (double)(predecessor ? x.first : n);
-            if (digits_pay(m, work[1], work[0], total, predecessor ? uq.back().first : n)) {
+            if (digits_pay(m, nfull, work[1], work[0], total, predecessor ? uq.back().first : n)) {
                 for (auto& x : uq) std::swap(x.first, x.second);
                 std::vector<int> bad;
                 int dstatus = 0;
