@@ -18,13 +18,16 @@
 //      by tcgen05.mma (kind::f16, M=128, N=256, K=16) and the epilogue turns it
 //      into certified bounds [dl2, du2] of the squared residual distance.  Each
 //      epilogue thread keeps the k smallest du2 of its row half in a heap; the
-//      k-th is an upper bound tau^2 of the true k-th distance, and every
-//      candidate with dl2 <= tau^2 (tau as it stands when the pair is seen) is
-//      kept.  The nearest-first warm-up makes tau tight before any pair is kept.
+//      k-th of the row's two heaps together is an upper bound tau^2 of the true
+//      k-th distance, and every candidate with dl2 <= tau^2 (tau as it stands
+//      when the pair is seen) is kept.  The nearest-first warm-up makes tau tight
+//      before any pair is kept.
 //   3. Rescore.  Each survivor's distance is recomputed from the f32 inputs with
-//      a compensated FP32 dot product (TwoProd/TwoSum) and an FP64 kernel value
-//      and normalisation; the k best (distance, index) pairs are written out.
-//      Queries whose survivor list overflowed are rescored exhaustively.
+//      a compensated FP32 dot product (TwoProd/TwoSum) and a double-float kernel
+//      value and normalisation; the k best (distance, index) pairs are written out.
+//      Queries whose survivor list overflowed are searched again over all their
+//      candidates: on the tensor cores with exact digit products (ct_digits.cuh),
+//      or, where they are few, by the general exhaustive kernels.
 //
 // Error bound of the screened dot (per pair), with u = 2^-8 (bf16) and
 // v = hi + lo + r, |r| <= u^2 |v|:  |s - v_q.v_c| <= c_split ||v_q|| ||v_c|| with
