@@ -701,14 +701,14 @@ def main():
     achieved = alg_flops / (screen_ms / 1e3) / 1e12
     # DRAM bytes per screened pair of the sweep, from a one-pass ncu capture of a full-size
     # launch of this workload, scaled to this launch's pairs
-    sweep_dram_bytes_per_pair = 11.39
+    sweep_dram_bytes_per_pair = 6.80
     roofline = {
         "bound": "tensor", "kernel": "screen_sweep_kernel (main sweep)", "achieved": achieved,
         "peak": bf16_sus, "unit": "TFLOP/s", "frac": achieved / bf16_sus,
         "traffic": sweep_dram_bytes_per_pair * pairs_main,
-        "traffic_note": "bytes per launch: 11.39 B per screened pair x pairs of this launch (ncu "
+        "traffic_note": "bytes per launch: 6.80 B per screened pair x pairs of this launch (ncu "
                         "dram__bytes_read.sum + dram__bytes_write.sum of one full-size sweep launch, one pass: "
-                        "423.4 GB for 3.718e10 pairs)",
+                        "245.0 GB for 3.601e10 pairs)",
         "peak_kind": f"bf16_tflops_sustained ({peak_kind})",
         "tensor_issued_tflops": issued_flops / (screen_ms / 1e3) / 1e12,
         "kernel_ms": screen_ms, "algorithmic_pairs": alg_pairs, "pairs_screened": pairs_main,
