@@ -31,7 +31,7 @@
 // pair of digits 0.75, with the kernel value in the exact distances' arithmetic 1.6, the epilogue not
 // overlapped.  The compensated FP32 kernels need 9 ms for the same queries.  Whole calls: that one 11.3 ms
 // before, 2.7 with this pass; n = 262144, m = 512, 1102 such queries 132 and 108; 4096 points against
-// n = 131072, m = 256, 55 such queries 5.5 and 4.0.
+// n = 131072, m = 256, 55 such queries 4.3 and 3.7.
 
 constexpr int DS = 5;                       // digits
 constexpr int DO = 6;                       // orders kept
@@ -109,21 +109,25 @@ __host__ __device__ inline size_t digit_offset(long long row, int col, int digit
 }
 
 // Digits of V rows in that layout, in tiles of tr: row r < rows is V row rowmap[r] (none:
-// row0 + r); negative entries and the rows up to rows_pad are zero.
+// row0 + r); negative entries and the rows up to rows_pad are zero.  A warp takes 16 rows x 16 columns, so
+// that a digit's 512 bytes are contiguous (n = 262144, m = 512: 0.29 ms, 6.5 TB/s; 1.2 with lanes along a row).
 __global__ void digit_split_kernel(const float* __restrict__ v, int m, const int* __restrict__ rowmap, long long row0,
                                    long long rows, long long rows_pad, int tr, const float* __restrict__ scale,
                                    bf16* __restrict__ out) {
     const float inv = 64.f / *scale;
-    const long long groups = m / 8, total = rows_pad * groups;
+    const int blocks = m / DK;
+    const long long total = rows_pad / 16 * blocks * 32;  // rows_pad: a multiple of 64
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const long long r = t / groups;
-        const int cg = (int)(t - r * groups);
+        const long long g = (t >> 5) / blocks;
+        const long long r = g * 16 + (t >> 4 & 1) * 8 + (t & 7);
+        const int col = (int)((t >> 5) - g * blocks) * DK + (int)(t >> 3 & 1) * 8;
         const int src = r >= rows ? -1 : rowmap ? rowmap[r] : (int)(row0 + r);
         float x[8];
+        load8(v, src, m, col, x);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = src >= 0 ? v[(size_t)src * m + cg * 8 + e] * inv : 0.f;  // exact scaling
-        const size_t off = digit_offset(r, cg * 8, 0, tr, m);
+        for (int e = 0; e < 8; ++e) x[e] *= inv;  // exact
+        const size_t off = digit_offset(r, col, 0, tr, m);
 #pragma unroll
         for (int s = 0; s < DS; ++s) {
             __align__(16) bf16 dg[8];

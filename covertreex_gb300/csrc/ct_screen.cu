@@ -867,28 +867,41 @@ __global__ void build_group_records_kernel(const int* __restrict__ ids, long lon
     }
 }
 
+// Eight columns of a V row (zeros for src < 0); 16-byte reads: V rows are the tree's own, m a multiple of 32.
+__device__ __forceinline__ void load8(const float* __restrict__ v, int src, int m, int col, float (&x)[8]) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4* p = (const float4*)(v + (size_t)(src < 0 ? 0 : src) * m + col);
+    const float4 a = src < 0 ? z : __ldg(p), b = src < 0 ? z : __ldg(p + 1);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+
 // hi/lo split of V rows into the blocked layout.  rowmap[r] = dataset row of
-// blocked row r (or -1 for a zero row).  One thread per (row, 8-column group).
+// blocked row r (or -1 for a zero row).
+// A warp takes 8 rows x 32 columns, one 512-byte block of either matrix, and the warps next to it the same
+// rows' next columns: reads are whole lines and writes contiguous (n = 262144, m = 512: 159 us, 6.7 TB/s; 461 with a thread per
+// row and 8 columns, lanes along the row).
 __global__ void split_blocked_kernel(const float* __restrict__ v, int m, const int* __restrict__ rowmap,
                                      long long rows_pad, bf16* __restrict__ hi, bf16* __restrict__ lo) {
-    const long long groups = (long long)m / 8;
-    const long long total = rows_pad * groups;
+    const int chunks = m / KC;
+    const long long total = rows_pad / 8 * chunks * 32;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        long long r = t / groups;
-        int cg = (int)(t - r * groups);
-        int src = rowmap ? rowmap[r] : (int)r;
+        const long long g = (t >> 5) / chunks;
+        const long long r = g * 8 + (t & 7);
+        const int col = (int)((t >> 5) - g * chunks) * KC + (int)((t >> 3) & 3) * 8;
+        const int src = rowmap ? rowmap[r] : (int)r;
+        float x[8];
+        load8(v, src, m, col, x);
         __align__(16) bf16 h8[8];
         __align__(16) bf16 l8[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            float x = src >= 0 ? v[(size_t)src * m + cg * 8 + e] : 0.f;
-            bf16 h = __float2bfloat16_rn(x);
-            float rem = x - __bfloat162float(h);
+            const bf16 h = __float2bfloat16_rn(x[e]);
             h8[e] = h;
-            l8[e] = __float2bfloat16_rn(rem);
+            l8[e] = __float2bfloat16_rn(x[e] - __bfloat162float(h));
         }
-        size_t off = blocked_offset(r, cg * 8, rows_pad / 8);
+        const size_t off = blocked_offset(r, col, rows_pad / 8);
         *(uint4*)(hi + off) = *(const uint4*)h8;
         *(uint4*)(lo + off) = *(const uint4*)l8;
     }
@@ -2554,12 +2567,12 @@ struct DigitRun {
 // 3e-7 per pair and column of V for slots that their FP32 filter serves and 6e-7 for the others, after a
 // latency that grows with the slots; the digit pass at 4.3e-8 after 200 us and the split of the dataset.
 // Both sides, general against digits (m = 256 unless given).  Points against n = 131072: 1024 of them, 53
-// slots overflowed, 1.77 ms against 2.07; 512, 2708 slots, 2.16 against 2.30; 4096, 154 slots, 4.32 against
-// 3.91; 2048 (RBF), 16157 slots, 28.3 against 5.3.  Rows: 500 of n = 65536 at m = 512 (RBF) 11.6 against
-// 2.4; 3000 at m = 128, 155 slots, 1.93 against 1.72; every row of 20000 at m = 96 (RBF) 39.9 against 7.9.
+// slots overflowed, 1.78 ms against 1.91; 512, 2708 slots, 2.16 against 2.08; 4096, 154 slots, 4.31 against
+// 3.73; 2048 (RBF), 16157 slots, 28.3 against 5.1.  Rows: 500 of n = 65536 at m = 512 (RBF) 11.6 against
+// 2.3; 3000 at m = 128, 155 slots, 1.97 against 1.69; every row of 20000 at m = 96 (RBF) 40.0 against 7.9.
 static bool digits_pay(int m, int nslots, double filtered, double plain, double total, long long rows) {
     return std::min(300.0, 3.0 * nslots) + m * (3e-7 * filtered + 6e-7 * plain) >
-           200.0 + 1.1e-5 * (double)rows * m + 4.3e-8 * m * total;
+           200.0 + 5e-6 * (double)rows * m + 4.3e-8 * m * total;
 }
 constexpr size_t kDigitSlabBytes = size_t(4) << 30;
 constexpr int kDigitBatch = 4096;      // rows per batch (their survivor lists are 32 KiB each)
