@@ -50,3 +50,17 @@ def test_digit_pass_repeated_rows_and_tiny_residuals(cuda_available):
     idx = CudaResidualIndex(V, p, X, variance=1.0, lengthscale=case["ls"], kernel_type=0, build_tree=False)
     q = np.concatenate([np.asarray(case["inducing"][:64]), np.arange(3000, 3040), np.arange(9000, 11000)])
     _check(idx, q.astype(np.int64), 20)
+
+
+def test_digit_pass_leaves_norms_without_a_scale_to_the_general_pass(cuda_available, monkeypatch):
+    """One V row whose squared norm overflows: no scale of the digits holds it."""
+    from covertreex_gb300.device import CudaResidualIndex
+
+    case = gaussian_case(24000, 3, 128, 1, 2.0, seed=5)
+    V = case["V"].copy()
+    V[777] = 1e20
+    idx = CudaResidualIndex(V, case["p"], case["X"], variance=1.0, lengthscale=case["ls"], kernel_type=1,
+                            build_tree=False)
+    monkeypatch.setenv("CT_SCREEN_SURVIVOR_CAP", "64")
+    q = np.random.default_rng(6).choice(np.delete(np.arange(24000), 777), 1500, replace=False).astype(np.int64)
+    _check(idx, q, 20)
