@@ -87,14 +87,13 @@ __host__ __device__ inline DigitSmem digit_smem() {
     return L;
 }
 
-// Scale of the search, from the largest row norm (so of every |v|) of the dataset and the queries.  Norms
-// that are not finite, or too large to square, give NaN: every bound is then NaN, which pass A ignores and
-// pass B keeps, so that the rows go to the general kernels.
+// Scale of the search, from the largest row norm (so of every |v|) of the dataset and the queries, which is
+// below kDigitMaxNorm (digit_fit).
 __global__ void digit_scale_kernel(const unsigned* __restrict__ vn_max, float* __restrict__ scale) {
     const float v = __uint_as_float(*vn_max);
     int e = 0;
-    if (v > 0.f && v < 1e15f) frexpf(v * 0.9924f, &e);  // v < 64.5 / 64 2^e: the leading digit is at most 64
-    *scale = v < 1e15f ? ldexpf(1.f, e > -50 ? e : -50) : __int_as_float(0x7fc00000);
+    if (v > 0.f) frexpf(v * 0.9924f, &e);  // v < 64.5 / 64 2^e: the leading digit is at most 64
+    *scale = ldexpf(1.f, e > -50 ? e : -50);
 }
 __global__ void gather_max_bits_kernel(const float* __restrict__ x, const int* __restrict__ rows, long long n,
                                        unsigned* __restrict__ out) {

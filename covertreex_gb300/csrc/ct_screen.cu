@@ -1572,17 +1572,35 @@ __global__ void merge_chunks_kernel(RescoreParams P, const int* item_begin, cons
     }
 }
 
-// Slots whose survivor lists overflowed; bit 31 marks those for the filtered pass.
+// Whether the digit pass's bounds of a row's pairs are numbers: a norm and coordinates whose squares and
+// products stay finite, and a 1/sqrt(p) that is neither NaN (p negative or NaN) nor 0 (p infinite).  One such
+// row makes bounds NaN, which no threshold test orders, so a call that meets one takes the general kernels.
+constexpr float kDigitMaxNorm = 1e15f;
+__device__ __forceinline__ bool digit_fit(const float* __restrict__ xs, int d, const float* __restrict__ vn,
+                                          const float* __restrict__ isp, long long r) {
+    bool ok = vn[r] < kDigitMaxNorm && isp[r] > 0.f;
+    for (int c = 0; c < d; ++c) ok = ok && fabsf(xs[(size_t)r * d + c]) < kDigitMaxNorm;
+    return ok;
+}
+__global__ void digit_unfit_kernel(const float* __restrict__ xs, int d, const float* __restrict__ vn,
+                                   const float* __restrict__ isp, long long n, int* __restrict__ unfit) {
+    const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (r < n && !digit_fit(xs, d, vn, isp, r)) atomicAdd(unfit, 1);
+}
+
+// Slots whose survivor lists overflowed; bit 31 marks those for the filtered pass.  counts: the slots listed,
+// (the survivor pass's), those whose query does not fit the digit pass.
 __global__ void collect_overflow_kernel(const int* __restrict__ surv_cnt, long long nslots, int half_cap,
-                                        const int* __restrict__ slot_id, const float* __restrict__ isp,
-                                        const float* __restrict__ vn, int filter, int* __restrict__ list,
-                                        int* __restrict__ nlist) {
+                                        const int* __restrict__ slot_id, const float* __restrict__ xs, int d,
+                                        const float* __restrict__ isp, const float* __restrict__ vn, int filter,
+                                        int* __restrict__ list, int* __restrict__ counts) {
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (s >= nslots) return;
     if (surv_cnt[2 * s] > half_cap || surv_cnt[2 * s + 1] > half_cap) {
         const int q = slot_id[s];
         const bool f = filter && q >= 0 && isp[q] * vn[q] <= kFilterIsq;
-        list[atomicAdd(nlist, 1)] = (int)s | (f ? (int)0x80000000u : 0);
+        list[atomicAdd(&counts[0], 1)] = (int)s | (f ? (int)0x80000000u : 0);
+        if (q >= 0 && !digit_fit(xs, d, vn, isp, q)) atomicAdd(&counts[2], 1);
     }
 }
 
@@ -1620,6 +1638,8 @@ struct State {
     float *rec_lvl = nullptr, *rec_ds = nullptr;  // sweep candidate records, tile order
     unsigned* xmax_max = nullptr;                 // bits of max |x| over the dataset rows
     unsigned* vn_max = nullptr;                   // bits of max ||v|| over the dataset rows
+    int* digit_unfit = nullptr;                   // dataset rows that do not fit the digit pass, and
+    int digit_unfit_rows = 0;                     // their number on the host
     double* inv_ls64 = nullptr;
     float* inv_ls_df = nullptr;             // (hi, lo) float pairs of 1 / lengthscale
     int* status = nullptr;
@@ -2758,6 +2778,7 @@ void ct_tree::release_screen() {
     cudaFree(S->lvl_hi); cudaFree(S->lvl_lo); cudaFree(S->lvl_id); cudaFree(S->lvl_key); cudaFree(S->lvl_meta);
     cudaFree(S->vn); cudaFree(S->isp); cudaFree(S->xmax); cudaFree(S->inv_ls64); cudaFree(S->status);
     cudaFree(S->inv_ls_df); cudaFree(S->isp_max); cudaFree(S->rec_ds); cudaFree(S->rec_lvl); cudaFree(S->xmax_max); cudaFree(S->vn_max);
+    cudaFree(S->digit_unfit);
     cudaFree(S->bounds);
     if (S->slab_done) cudaEventDestroy(S->slab_done);
     delete S;
@@ -2802,6 +2823,7 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
     A((void**)&S->isp_max, sizeof(unsigned));
     A((void**)&S->xmax_max, sizeof(unsigned));
     A((void**)&S->vn_max, sizeof(unsigned));
+    A((void**)&S->digit_unfit, sizeof(int));
     A((void**)&S->rec_ds, sizeof(float) * RT * (S->rows_pad / TC));
     A((void**)&S->rec_lvl, sizeof(float) * RT * (S->lvl_rows / TC));
     A((void**)&S->inv_ls64, sizeof(double) * 64);
@@ -2824,6 +2846,8 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
         if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->xmax, n, S->xmax_max);
         if (e == cudaSuccess) e = cudaMemsetAsync(S->vn_max, 0, sizeof(unsigned), st);
         if (e == cudaSuccess) max_bits_kernel<<<grid_for(n), 256, 0, st>>>(S->vn, n, S->vn_max);
+        if (e == cudaSuccess) e = cudaMemsetAsync(S->digit_unfit, 0, sizeof(int), st);
+        if (e == cudaSuccess) digit_unfit_kernel<<<grid_for(n), 256, 0, st>>>(T->xs, T->d, S->vn, S->isp, n, S->digit_unfit);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     std::vector<long long> meta;
@@ -2862,6 +2886,8 @@ static int screen_prepare(ct_tree* T, cudaStream_t st) {
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(S->inv_ls_df, ils_df, sizeof(float) * 2 * T->d, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(S->status, 0, sizeof(int), st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&S->digit_unfit_rows, S->digit_unfit, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // host vectors above go out of scope
     }
     if (e != cudaSuccess) return T->set_err(CT_ERR_CUDA, "screen prep: %s", cudaGetErrorString(e));
@@ -2913,7 +2939,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     A((void**)&hist, sizeof(unsigned) * 256 * (size_t)nbh);
     A((void**)&a_slot_lvl, sizeof(int) * rows_q);
     A((void**)&rowmap_lvl, sizeof(int) * rows_q);
-    A((void**)&nfull_d, 2 * sizeof(int));  // overflowed slots; slots of the survivor pass's second kernel
+    A((void**)&nfull_d, 3 * sizeof(int));  // overflowed slots; slots of the survivor pass's second kernel; unfit ones
     A((void**)&evals_d, sizeof(long long));
     A((void**)&qtau, sizeof(unsigned) * nq);
     if (e != cudaSuccess) return set_err(CT_ERR_NOMEM, "screened form allocation: %s", cudaGetErrorString(e));
@@ -3120,7 +3146,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         e = cudaMemcpyAsync(unit_jobs_d, unit_jobs_h.data(), sizeof(int2) * unit_jobs_h.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(unit_counter, 0, sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(surv_cnt, 0, sizeof(int) * 2 * nslots, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(nfull_d, 0, 2 * sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(nfull_d, 0, 3 * sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(evals_d, 0, sizeof(long long), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(S->status, 0, sizeof(int), st);
     // ---- sweep
@@ -3167,16 +3193,17 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     R.big_list = big_list; R.big_cnt = nfull_d + 1;
     // The overflow list first: the exhaustive pass is planned on the host and runs on side
     // streams while the survivor pass runs on the call's stream.
-    int nfull = 0, status = 0;
+    int nfull = 0, unfit = 0, status = 0;
     long long exh_pairs = 0;  // candidates of the exhaustive pass (part tiles count whole tiles)
     cudaEvent_t ev_ovf = nullptr;
     if (e == cudaSuccess) {
-        collect_overflow_kernel<<<grid_for(nslots), 256, 0, st>>>(surv_cnt, nslots, half_cap, slot_id_use, S->isp, S->vn,
-                                                                    can_filter ? 1 : 0, full_list, nfull_d);
+        collect_overflow_kernel<<<grid_for(nslots), 256, 0, st>>>(surv_cnt, nslots, half_cap, slot_id_use, xs, d, S->isp,
+                                                                    S->vn, can_filter ? 1 : 0, full_list, nfull_d);
         e = cudaGetLastError();
         ++launches;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nfull, nfull_d, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&unfit, nfull_d + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&status, S->status, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_ovf, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventRecord(ev_ovf, st);
@@ -3226,8 +3253,10 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         auto slot_of = [](int v) { return v & 0x7fffffff; };
         auto filt_of = [](int v) { return v < 0 ? 1 : 0; };
         // The digit pass takes every query with an overflowed slot, over all its candidates; what its
-        // rows cannot hold stays for the kernels below.
-        if (e == cudaSuccess && m <= kDigitMaxM) {
+        // rows cannot hold stays for the kernels below, and so does every slot where a row of the dataset or
+        // an overflowed query would give it bounds that are not numbers (digit_fit).
+        if (e == cudaSuccess && m <= kDigitMaxM && S->digit_unfit_rows == 0 && unfit == 0 && var >= 0.f &&
+            var <= CT_FLT_MAX) {
             std::vector<std::pair<int, int>> uq;  // (dataset id, query of the call)
             double work[2] = {0, 0}, total = 0;   // pairs of the slots, plain and filtered; of their queries
             for (int i = 0; i < nfull; ++i) {

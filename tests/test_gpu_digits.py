@@ -5,6 +5,7 @@ from the same double-float dot and kernel value, so the rows agree bit for bit.
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from tests._data import gaussian_case, mixture_case
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +65,75 @@ def test_digit_pass_leaves_norms_without_a_scale_to_the_general_pass(cuda_availa
     monkeypatch.setenv("CT_SCREEN_SURVIVOR_CAP", "64")
     q = np.random.default_rng(6).choice(np.delete(np.arange(24000), 777), 1500, replace=False).astype(np.int64)
     _check(idx, q, 20)
+
+
+def _check_healthy_rows(case, bad, q, gi, k, predecessor):
+    """Neighbours other than the rows `bad` against the FP64 search over the rest: a row whose distances are
+    not numbers takes no other row's place but its own."""
+    n = len(case["p"])
+    keep = np.delete(np.arange(n), bad)
+    rank = np.cumsum(np.isin(np.arange(n), bad, invert=True)) - 1
+    V, p, X = case["V"][keep], case["p"][keep], case["X"][keep]
+    kk = k - len(bad)
+    ri, _ = O.brute_knn_f64(V, p, X, 1.0, case["ls"], case["kt"], rank[q], kk, predecessor)
+    got = np.full((len(q), kk), -1, np.int64)
+    for r in range(len(q)):
+        g = gi[r][(gi[r] >= 0) & ~np.isin(gi[r], bad)][:kk]
+        got[r, :g.size] = rank[g]
+    assert np.array_equal(got >= 0, ri >= 0)
+
+    def dist_fn(r, ids):
+        return O.residual_dist_f64(V, p, X, 1.0, case["ls"], case["kt"], np.array([rank[q[r]]]), ids)[0]
+
+    _, mism = O.near_tie_mismatches(got, ri, dist_fn)
+    assert not [t for t in mism if t[3] >= 1e-6]
+
+
+# Rows of at most 2 x 2048 candidates: their survivor lists hold every candidate, so nothing but the
+# pass's own rules can send them to the general kernels.
+SHORT_ROWS = [(3000, 0, 3000, False), (24000, 1024, 4096, True)]
+
+
+@pytest.mark.parametrize("n,lo,hi,predecessor", SHORT_ROWS)
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e20])
+def test_digit_pass_short_rows_beside_a_row_without_a_scale(cuda_available, monkeypatch, n, lo, hi, predecessor, value):
+    from covertreex_gb300.device import CudaResidualIndex
+
+    case = gaussian_case(n, 3, 128, 1, 2.0, seed=5)
+    V = case["V"].copy()
+    V[777] = value
+    idx = CudaResidualIndex(V, case["p"], case["X"], variance=1.0, lengthscale=case["ls"], kernel_type=1,
+                            build_tree=False)
+    monkeypatch.setenv("CT_SCREEN_SURVIVOR_CAP", "64")
+    ids = np.delete(np.arange(n), 777)
+    ids = ids[(ids >= lo) & (ids < hi)]
+    q = np.sort(np.random.default_rng(6).choice(ids, 1500, replace=False)).astype(np.int64)
+    gi, _ = idx.knn(q, 20, predecessor=predecessor, form="screened")
+    assert idx.last_stats["overflow_queries"] > 0
+    _check_healthy_rows(case, [777], q, gi, 20, predecessor)
+
+
+@pytest.mark.parametrize("n,lo,hi,predecessor", SHORT_ROWS)
+def test_digit_pass_short_rows_beside_residuals_without_a_root(cuda_available, monkeypatch, n, lo, hi, predecessor):
+    """Negative, NaN and zero p: the pair's normalisation is the floor, so that such a row lies at distance 0
+    of every query that is searched exhaustively; 1 / sqrt(p) is no number or infinite."""
+    from covertreex_gb300.device import CudaResidualIndex
+
+    case = gaussian_case(n, 3, 128, 1, 2.0, seed=5)
+    bad = [100, 777, 1000]
+    p = case["p"].copy()
+    p[bad] = [-0.25, np.nan, 0.0]
+    idx = CudaResidualIndex(case["V"], p, case["X"], variance=1.0, lengthscale=case["ls"], kernel_type=1,
+                            build_tree=False)
+    monkeypatch.setenv("CT_SCREEN_SURVIVOR_CAP", "64")
+    ids = np.delete(np.arange(n), bad)
+    ids = ids[(ids >= lo) & (ids < hi)]
+    q = np.sort(np.random.default_rng(6).choice(ids, 1500, replace=False)).astype(np.int64)
+    gi, _ = idx.knn(q, 20, predecessor=predecessor, form="screened")
+    assert idx.last_stats["overflow_queries"] > 0
+    _check_healthy_rows(case, bad, q, gi, 20, predecessor)
+    if n == 3000:  # one candidate part: an overflowed query is searched over all rows, the others are screened,
+        # which leaves rows without a number out
+        listed = np.isin(gi, [100, 777]).sum(axis=1)
+        assert np.all((listed == 0) | (listed == 2))
+        assert np.count_nonzero(listed == 2) == idx.last_stats["overflow_queries"]
