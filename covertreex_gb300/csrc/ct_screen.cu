@@ -911,14 +911,14 @@ __global__ void split_blocked_kernel(const float* __restrict__ v, int m, const i
 // sums the squares in FP32, every step rounded up (an upper bound of ||v|| within
 // (m / 32 + 5) 2^-23 of it), then each lane finishes a row (the FP64 reciprocal root of p costs a
 // warp as much for one lane as for 32).  65536 rows of 256: 12 us; 64 us as one strided FP64
-// chain per thread.
+// chain per thread.  Norms above 1.8e19, whose square FP32 does not hold, are summed in FP64.
 __global__ void point_scalars_kernel(const float* __restrict__ v, const float* __restrict__ p,
                                      const float* __restrict__ xs, long long n, int m, int d, float* __restrict__ vn,
                                      float* __restrict__ isp, float* __restrict__ xmax) {
     const long long r0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) & ~31LL;
     const int lane = threadIdx.x & 31;
     const int rows = r0 < n ? (int)(n - r0 < 32 ? n - r0 : 32) : 0;
-    float mine = 0.f;
+    float mine = 0.f, wide = 0.f;
     for (int i = 0; i < rows; ++i) {
         const float* row = v + (size_t)(r0 + i) * m;
         float s = 0.f;
@@ -926,10 +926,17 @@ __global__ void point_scalars_kernel(const float* __restrict__ v, const float* _
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s = __fadd_ru(s, __shfl_xor_sync(0xffffffffu, s, o));
         if (lane == i) mine = s;
+        if (!(s <= CT_FLT_MAX)) {  // (s is the same in every lane)
+            double t = 0.0;
+            for (int c = lane; c < m; c += 32) t += (double)row[c] * row[c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == i) wide = __double2float_ru(sqrt(t) * (1.0 + 1e-12));
+        }
     }
     const long long r = r0 + lane;
     if (r >= n) return;
-    vn[r] = __fsqrt_ru(mine);
+    vn[r] = mine <= CT_FLT_MAX ? __fsqrt_ru(mine) : wide;
     isp[r] = (float)(1.0 / sqrt((double)p[r]));
     float mx = 0.f;
     for (int c = 0; c < d; ++c) mx = fmaxf(mx, fabsf(xs[(size_t)r * d + c]));

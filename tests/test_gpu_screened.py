@@ -152,3 +152,20 @@ def test_screened_forced_exhaustive_pass_vs_fp64(cuda_available, monkeypatch, pr
     hi, hd = idx.knn(q, 40, predecessor=predecessor, form="screened")
     assert idx.last_stats["overflow_queries"] < st["overflow_queries"]
     assert np.array_equal(hi, gi) and np.array_equal(hd.view(np.uint32), gd.view(np.uint32))
+
+
+@pytest.mark.parametrize("value", [1e20, 3e36])
+def test_screened_query_with_a_huge_norm_among_zero_rows(cuda_available, value):
+    """Norms whose square passes the FP32 range, against rows of V that are exactly zero: the dot's error
+    term is norm times zero, so that the kernel value alone decides."""
+    n, m, q0 = 3000, 64, 5
+    r = np.random.default_rng(31)
+    X = r.standard_normal((n, 3)).astype(np.float32)
+    V = np.zeros((n, m), np.float32)
+    V[q0] = value / 8
+    case = dict(V=V, p=r.uniform(0.5, 1.0, n).astype(np.float32), X=X, var=1.0, ls=np.full(3, 1.0, np.float32), kt=1)
+    idx = _index(case)
+    for q in (np.array([q0]), np.arange(n)):
+        gi, gd = idx.knn(q, 20, form="screened")
+        row = int(np.flatnonzero(q == q0)[0])
+        _check_against_fp64(case, q[[row]], 20, False, gi[[row]], gd[[row]])
