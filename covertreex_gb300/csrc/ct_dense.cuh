@@ -115,7 +115,7 @@ struct Smem {
     size_t a, b, buf, list, tau, thr, xq, nq, pq, qid, cnt, cand, pend, npend, total;
 };
 
-__host__ __device__ inline Smem layout(int cfg, int m, int d, int k, int ns, int wmax, int slack) {
+__host__ __device__ inline Smem layout(int cfg, int m, int d, int k, int ns, int wmax, int slack, int pend) {
     Smem L;
     const int qt = cfg_qt(cfg), ct = cfg_ct(cfg);
     const Geo g = geometry(m, wmax);
@@ -133,23 +133,26 @@ __host__ __device__ inline Smem layout(int cfg, int m, int d, int k, int ns, int
     L.qid = take(sizeof(int) * qt);
     L.cnt = take(sizeof(int) * qt);
     L.cand = take(sizeof(float) * cand_buffers(g) * ct * (d + 2));
-    L.pend = take((sizeof(float) + sizeof(int)) * kPend);
+    L.pend = take((sizeof(float) + sizeof(int)) * pend);
     L.npend = take(2 * sizeof(int));
     L.total = off;
     return L;
 }
 
-// Ring depth, stage width and buffer slack of a configuration at (m, d, k): the deepest ring and
-// roomiest buffers that fit `limit` bytes (a query's buffer holds CT + slack keys and is merged
-// above `slack`); narrow stages are the 16-row forms' last resort.  False when nothing fits.
+// Ring depth, stage width, buffer slack and pending pairs of a configuration at (m, d, k): the deepest
+// ring and roomiest buffers that fit `limit` bytes (a query's buffer holds CT + slack keys and is merged
+// above `slack`); narrow stages are the 16-row forms' last resort, and a short list of pending pairs
+// their last (m = 1936 to 1968 with more than 50 coordinates; pairs past it are evaluated in place).
+// False when nothing fits.
 struct Ring {
-    int ns, wmax, slack;
+    int ns, wmax, slack, pend;
 };
 __host__ inline bool pick_ring(int cfg, int m, int d, int k, size_t limit, Ring* r, size_t* total) {
-    const Ring tries[7] = {{3, 64, 32}, {3, 64, 16}, {2, 64, 16}, {2, 64, 8}, {2, 64, 4}, {2, 16, 16}, {2, 16, 4}};
+    const Ring tries[8] = {{3, 64, 32, kPend}, {3, 64, 16, kPend}, {2, 64, 16, kPend}, {2, 64, 8, kPend},
+                           {2, 64, 4, kPend},  {2, 16, 16, kPend}, {2, 16, 4, kPend},  {2, 16, 4, 64}};
     for (const Ring& t : tries) {
         if (t.wmax == 16 && cfg_qt(cfg) != 16) continue;
-        const size_t need = layout(cfg, m, d, k, t.ns, t.wmax, t.slack).total;
+        const size_t need = layout(cfg, m, d, k, t.ns, t.wmax, t.slack, t.pend).total;
         if (need <= limit) {
             *r = t;
             *total = need;
@@ -436,7 +439,8 @@ __device__ __noinline__ void run_tile_v(const Tile& P, u64 nz) {
     static_assert(WQ * (CT / (8 * CPT)) == kWarps, "warps cover the tile");
     constexpr int STR = stage_stride(WMAX);
     const int ns = P.ring.ns, slack = P.ring.slack, CAP = CT + slack;
-    const Smem S = layout(C, P.m, P.d, P.k, ns, WMAX, slack);
+    const int pend = WMAX == 16 ? P.ring.pend : kPend;
+    const Smem S = layout(C, P.m, P.d, P.k, ns, WMAX, slack, pend);
     const Geo g = geometry(P.m, WMAX);
     const int ncand = cand_buffers(g);
     float* As = (float*)(smem_raw + S.a);
@@ -452,7 +456,7 @@ __device__ __noinline__ void run_tile_v(const Tile& P, u64 nz) {
     int* Cnt = (int*)(smem_raw + S.cnt);
     float* Cand = (float*)(smem_raw + S.cand);
     float* PendDot = (float*)(smem_raw + S.pend);
-    int* PendPair = (int*)(PendDot + kPend);
+    int* PendPair = (int*)(PendDot + pend);
     int* Npend = (int*)(smem_raw + S.npend);
 
     const int tid = threadIdx.x;
@@ -795,7 +799,7 @@ __device__ __noinline__ void run_tile_v(const Tile& P, u64 nz) {
                 if (lane == 0) at = atomicAdd(npend, __popc(who));
                 at = __shfl_sync(0xffffffffu, at, 0) + __popc(who & ((1u << lane) - 1u));
                 if (mine) {
-                    if (at < kPend) {
+                    if (at < pend) {
                         PendDot[at] = h[a][b];
                         PendPair[at] = (qrow + 4 * a) << 16 | (crow + 8 * b);
                     } else {
@@ -804,7 +808,7 @@ __device__ __noinline__ void run_tile_v(const Tile& P, u64 nz) {
                 }
             }
         __syncthreads();
-        const int np = min(*npend, kPend);
+        const int np = min(*npend, pend);
         if (tid == 0) Npend[(t & 1) ^ 1] = 0;
         if (np > 0) {
             for (int i = tid; i < np; i += kThreads) {

@@ -72,3 +72,35 @@ def test_variance_scales_the_skip_test(cuda_available, kt, var):
     gi, gd = index.knn(q, 30, form="dense")
     oi, od = O.brute_knn_f32(V, p, X, var, ls, kt, q, 30, False)
     assert np.array_equal(gi, oi) and np.array_equal(gd.view(np.uint32), od.view(np.uint32))
+
+
+@pytest.mark.parametrize("m,d,k", [(1936, 51, 113), (1936, 64, 80), (1952, 64, 68), (1968, 64, 56), (1936, 3, 128)])
+@pytest.mark.parametrize("pred", [False, True])
+def test_widest_rows_with_many_coordinates(cuda_available, m, d, k, pred):
+    """The largest shared-memory needs of the 16-row tile, through the id, batch and allocation-free entry points."""
+    import torch
+
+    from covertreex_gb300 import _lib
+    from covertreex_gb300.device import CudaBatch, CudaResidualIndex
+    from tests.test_zz_no_alloc import _noalloc
+
+    V, p, X = _case(300, d, m, m + d + k)
+    ls = np.full(d, 2.0, np.float32)
+    q = np.arange(0, 300, 7)
+    index = CudaResidualIndex(V, p, X, variance=1.0, lengthscale=ls, kernel_type=1, build_tree=False)
+    oi, od = O.brute_knn_f32(V, p, X, 1.0, ls, 1, q, k, pred)
+    batch = CudaBatch()
+    bi, bd = batch.add_ids(index, q, k, predecessor=pred)
+    batch.run()
+    rc, ni, nd = _noalloc(_lib.load(), dict(V=V, p=p, X=X, var=1.0, ls=ls, kt=1), q, k, pred, torch,
+                          torch.cuda.current_stream())
+    assert rc == 0
+    for gi, gd in (index.knn(q, k, predecessor=pred, form="dense"), (bi.cpu().numpy(), bd.cpu().numpy()), (ni, nd)):
+        assert np.array_equal(gi, oi) and np.array_equal(gd.view(np.uint32), od.view(np.uint32))
+
+
+@pytest.mark.parametrize("m,d,k", [(1936, 51, 115), (1936, 64, 83), (1952, 64, 71), (1968, 64, 59)])
+def test_widest_rows_of_the_single_tree_form(cuda_available, m, d, k):
+    """The last sizes the 227 KB of a block hold (the batch kernel's own scalars leave it a little less)."""
+    V, p, X = _case(300, d, m, m + d + k)
+    _check(V, p, X, 1, 2.0, np.arange(0, 300, 7), k, False)
