@@ -21,6 +21,7 @@
 // the GEMM is register-tiled 64 x 64 with 4 x 4 outputs per thread and is bound by
 // the DFMA rate; N m^2 FMAs for N rows.
 #include <cuda_runtime.h>
+#include <float.h>
 
 #include <algorithm>
 #include <math.h>
@@ -56,6 +57,7 @@ __device__ __forceinline__ double kernel_f64(const double* __restrict__ x, const
 inline double2 scale_of(int kt, double ls) {
     const double denom = ls > 1e-12 ? ls : 1e-12;
     const double b = kt == 1 ? denom : denom * denom;
+    if (b > DBL_MAX) return make_double2(1.0, 0.0);  // x / inf: div_by(x, 1, 0) is 0 for every finite x
     return make_double2(b, 1.0 / b);
 }
 

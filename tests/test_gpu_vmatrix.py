@@ -152,3 +152,12 @@ def test_concurrent_embeds_on_one_factor(cuda_available):
         t.join()
     f.free()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("kt", [0, 1])
+@pytest.mark.parametrize("ls", [1e160, np.inf])
+def test_vmatrix_of_a_constant_kernel(cuda_available, kt, ls):
+    """A lengthscale whose square, or which itself, is infinite: every scaled distance is 0."""
+    X = np.random.default_rng(9).standard_normal((700, 3))
+    V, p = _check(X.astype(np.float32), 40, kt, ls)
+    assert np.all(np.isfinite(V)) and np.all(np.isfinite(p))
