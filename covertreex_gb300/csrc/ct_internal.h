@@ -9,6 +9,11 @@ namespace ct {
 // per-thread timing switch (ct_set_timing)
 bool timing_enabled();
 
+// Priority of a call's side streams: one level above the stream of the call (numbers fall as priority
+// rises), where the device has one.  A pass that runs beside the call's own kernels starts ahead of their
+// queued blocks, and everything that the caller ranks at least two levels higher still goes first.
+inline int side_stream_priority(int call, int greatest) { return call > greatest ? call - 1 : greatest; }
+
 struct BruteParams {
     const float* vperm;   // n x m, the dense tile's column order (see ct_setup.cu)
     const float* xs;      // n x d scaled coordinates

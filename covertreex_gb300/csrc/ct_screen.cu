@@ -3231,10 +3231,12 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     DigitRun digits;
     int nexh = nfull;  // slots left to the exhaustive kernels
     if (e == cudaSuccess && nfull > 0) {
-        // above the call's stream: the survivor pass fills the chip with short blocks, and a pass that
+        // one level above the call's stream: the survivor pass fills the chip with short blocks, and a pass that
         // started behind it would run after it (vecchia 32768 / 256: 6.57 ms, with priority 5.84)
-        int prio = 0, prio_least = 0;
-        cudaDeviceGetStreamPriorityRange(&prio_least, &prio);
+        int prio = 0, least = 0, greatest = 0;
+        e = cudaStreamGetPriority(st, &prio);
+        if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        prio = ct::side_stream_priority(prio, greatest);
         for (auto& a : aux)
             if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&a, cudaStreamNonBlocking, prio);
         for (auto& v : ev_aux)

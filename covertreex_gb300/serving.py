@@ -149,10 +149,11 @@ class ServingEngine:
         self.peak_bytes = 0
         self.rejected: set = set()
         self.evicted: set = set()
-        # Three stream priorities: dense steps (short, latency-bound) highest, screened
-        # requests next, builds lowest, so the block scheduler hands freed SMs to queued
-        # step kernels first and to build kernels last (p99 at 500 req/s 6.7-8.3 -> 6.1-6.4
-        # ms against one query priority).
+        # Stream priorities: dense steps (short, latency-bound) highest, screened requests
+        # two levels below (a screened call runs its exhaustive pass one level above its own
+        # stream), builds lowest, so the block scheduler hands freed SMs to queued step
+        # kernels first and to build kernels last (p99 at 500 req/s 6.7-8.3 -> 6.1-6.4 ms
+        # against one query priority).
         self.streams = [torch.cuda.Stream(self.device, priority=-3) for _ in range(slots)]
         self.batches = [CudaBatch(self.device) for _ in range(slots)]
         for b in self.batches:
@@ -167,7 +168,7 @@ class ServingEngine:
                          for st in self.build_streams]
         for w in self._workers:
             w.start()
-        self.screen_stream = torch.cuda.Stream(self.device, priority=-2)
+        self.screen_stream = torch.cuda.Stream(self.device, priority=-1)
         self._screen_in: "queue.Queue" = queue.Queue()
         self._screen_out: "queue.Queue" = queue.Queue()
         self._screener = threading.Thread(target=self._screened_worker, daemon=True)

@@ -109,3 +109,17 @@ def test_serving_budget_admission_and_eviction(cuda_available):
         assert len(eng.evicted) >= 1
     finally:
         eng.close()
+
+
+def test_serving_streams_leave_a_level_for_the_exhaustive_pass(cuda_available):
+    """A screened call's side streams run one level above its stream (ct_internal.h): still below the dense
+    steps, and above the builds."""
+    from covertreex_gb300.serving import ServingEngine
+
+    eng = ServingEngine(hbm_budget_bytes=1e9)
+    try:
+        side = eng.screen_stream.priority - 1
+        assert all(s.priority < side for s in eng.streams)
+        assert all(side < eng.screen_stream.priority < s.priority for s in eng.build_streams)
+    finally:
+        eng.close()
