@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "ct_common.cuh"
+#include "ct_fastmath.cuh"
 #include "ct_internal.h"
 #include "ct_sm100.cuh"
 #include "ct_tree.h"
@@ -190,30 +191,6 @@ __device__ __forceinline__ void heap_push(float* h, int n, float x) {
         i = pnt;
     }
     h[i * kEpiThreads] = x;
-}
-
-// e^x as ex2.approx of x log2(e), results below 2^-126 flushed to zero (__expf's own two steps without
-// its scaling of tiny results, whose 1e-38 the bounds' absolute 1e-30 covers).
-__device__ __forceinline__ float ex2_ftz(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float2 exp2x(float2 x) {
-    const float2 t = __fmul2_rn(x, make_float2(1.4426950408889634f, 1.4426950408889634f));
-    return make_float2(ex2_ftz(t.x), ex2_ftz(t.y));
-}
-// sqrt(x), x >= 0: s = x rsqrt(x) and one correction step, within 2^-45 relative before its last
-// rounding (half an ulp, as the bounds assume), without the branches of the IEEE routine.
-// 1e-15 for x = 0.
-__device__ __forceinline__ float2 sqrt2x(float2 x) {
-    x = make_float2(fmaxf(x.x, 1e-30f), fmaxf(x.y, 1e-30f));
-    float2 r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
-    const float2 s = __fmul2_rn(x, r);
-    const float2 e = __ffma2_rn(make_float2(-s.x, -s.y), s, x);
-    return __ffma2_rn(e, __fmul2_rn(r, make_float2(0.5f, 0.5f)), s);
 }
 
 // Squared scaled distance and kernel value of one query with two staged candidates
@@ -567,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_sweep_kernel(MMAParams P) 
             // kmax: an upper bound of the kernel value phase 1 computes for this row and any
             // candidate of its half tile.  The half tile's box gives the smallest squared
             // scaled distance dmin; phase 1's f32 distance (rounded differences, FMA chain) is
-            // at least dmin (1 - 1e-5), and its __expf / Matern polynomial stay within the
+            // at least dmin (1 - 1e-5), and its exponential / Matern polynomial stay within the
             // relative margins below.
             float kmax = 0.f;
             if (MODE == MODE_SWEEP && qid >= 0) {
@@ -1267,7 +1244,7 @@ template <int BUF = RBUF>
 __device__ __forceinline__ void warp_topk_append(unsigned long long* keys, int& fill, int k, bool has,
                                                  unsigned long long key);
 
-// Plain FP32 dots of the query slice with NC candidate rows (the split of warp_dots,
+// Plain FP32 dots of the query slice with four candidate rows (the split of warp_dots4,
 // one FMA per element, then a butterfly sum).  Each lane's chain has m/32 roundings
 // and the butterfly 5 more, so |error| <= (m/32 + 7) 2^-24 |v_q| |v_c|.
 template <int PER>
@@ -1886,7 +1863,7 @@ __global__ void __launch_bounds__(256) rescore_tile_kernel(RescoreParams P, cons
         const int cid = cid_s[lane];
         const bool va = ida >= 0 && cid >= 0 && (!P.predecessor || cid < ida);
         const bool vb = idb >= 0 && cid >= 0 && (!P.predecessor || cid < idb);
-        // The dot in warp_dots' order, so that a pair's exact distance is the same whichever
+        // The dot in warp_dots4's order, so that a pair's exact distance is the same whichever
         // pass scores it: 32 segments of m/32 elements, each summed in order, combined as
         // the butterfly does (lane offsets 16, 8, 4, 2, 1).  Taking segment rev5(c) at step
         // c turns that tree into a binary counter: pend[L] holds the finished subtree of

@@ -26,19 +26,11 @@
 #include <algorithm>
 #include <math.h>
 
+#include "ct_fastmath.cuh"
 #include "ct_vmatrix.h"
 
 namespace ct {
 namespace vmat {
-
-// x / b, correctly rounded, from y = the correctly rounded 1 / b: q = x y, then one residual step
-// (Markstein's theorem: three operations where the general division takes about twelve, on a chip
-// with two FP64 operations a clock per SM).  An infinite or NaN quotient is returned as it is.
-__device__ __forceinline__ double div_by(double x, double b, double y) {
-    const double q = x * y;
-    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return q;
-    return fma(fma(-b, q, x), y, q);
-}
 
 // Kernel value; ls2 = {max(ls, 1e-12), 1 / it} for Matern, {its square, 1 / that} for RBF.
 __device__ __forceinline__ double kernel_f64(const double* __restrict__ x, const double* __restrict__ z, int d,
