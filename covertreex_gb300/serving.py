@@ -126,6 +126,18 @@ def estimate_tree_bytes(n: int, d: int, m: int) -> int:
     return int(metric + screened + factor + transient)
 
 
+SLAB_POINTS = 4096  # new points of a screened request that a tree's query slab holds (CT_BUILD_QUERY_SLAB)
+
+
+def screened_workspace_bytes(n: int, m: int) -> int:
+    """Device bytes that a screened call's tensor-core exhaustive pass may take and its memory pool then
+    keeps: the dataset's digits (10 bytes per element of V, in slabs of at most 4 GiB), and for a batch of
+    4096 queries their digits and survivor lists (32 KiB each)."""
+    if m > 800:  # the pass's limit; the general kernels need little
+        return 0
+    return int(min(4 << 30, 10 * n * m) + SLAB_POINTS * (10 * m + (32 << 10)))
+
+
 class ServingEngine:
     def __init__(self, *, hbm_budget_bytes: float = 120e9, slots: int = 3, max_step_points: int = 16384,
                  max_step_work: float = 2.0e10, dense_pair_limit: float = 1.0e10, device=None,
@@ -230,8 +242,21 @@ class ServingEngine:
         self.used_bytes += tree.nbytes
         self.peak_bytes = max(self.peak_bytes, self.used_bytes + self.reserved_bytes)
 
-    def _evict_for(self, need: int, protect: set) -> bool:
-        while self.used_bytes + self.reserved_bytes + need > self.budget:
+    def _workspace(self, n: int, m: int) -> int:
+        """Workspace of one screened call (they run one at a time) on the resident trees or a tree of n x m;
+        0 where the largest request runs dense."""
+        return max(screened_workspace_bytes(a, b) if SLAB_POINTS * a * b > self.dense_pair_limit else 0
+                   for a, b in [(n, m)] + [(t.n, t.m) for t in self.trees.values()])
+
+    def _over_budget(self, need: int, n: int, m: int) -> bool:
+        held = self.used_bytes + self.reserved_bytes
+        # a tree that has the device to itself is admitted up to the whole budget: a screened call that
+        # finds no room for its workspace takes kernels that need little
+        return held + need > self.budget or (held > 0 and held + need + self._workspace(n, m) > self.budget)
+
+    def _evict_for(self, need: int, protect: set, n: int, m: int) -> bool:
+        """Make room for a tree of n x m that needs `need` bytes beside the screened workspace."""
+        while self._over_budget(need, n, m):
             idle = [t for t in self.trees.values() if t.inflight == 0 and t.rid not in protect]
             if not idle:
                 return False
@@ -412,7 +437,8 @@ class ServingEngine:
             if builds_inflight < len(self._workers) and pending_builds:
                 req = pending_builds[0]
                 n, d = req.coords.shape
-                est = estimate_tree_bytes(n, d, min(req.inducing_count, n))
+                m = min(req.inducing_count, n)
+                est = estimate_tree_bytes(n, d, m)
                 protect = {q.tree for q in pending_queries}
                 if est > self.budget:
                     pending_builds.pop(0)
@@ -421,7 +447,7 @@ class ServingEngine:
                     self.rejected.add(req.rid)
                     left -= 1
                     progressed = True
-                elif self._evict_for(est, protect):
+                elif self._evict_for(est, protect, n, m):
                     pending_builds.pop(0)
                     rec = recs[req.rid]
                     rec.start = now
@@ -505,7 +531,8 @@ class ServingEngine:
             if isinstance(r, BuildRequest):
                 rec = RequestRecord(r.rid, "build", r.arrival, r.coords.shape[0], start=time.perf_counter() - t0)
                 n, d = r.coords.shape
-                if not self._evict_for(estimate_tree_bytes(n, d, min(r.inducing_count, n)), set()):
+                m = min(r.inducing_count, n)
+                if not self._evict_for(estimate_tree_bytes(n, d, m), set(), n, m):
                     rec.status = "rejected"
                 else:
                     self._install(self._build_tree(r))
@@ -573,4 +600,4 @@ def latency_by_size(records: List[RequestRecord], kind: str = "query",
 
 
 __all__ = ["BuildRequest", "QueryRequest", "RequestRecord", "ServingEngine", "estimate_tree_bytes",
-           "latency_by_size", "latency_summary"]
+           "latency_by_size", "latency_summary", "screened_workspace_bytes"]
