@@ -137,3 +137,26 @@ def test_digit_pass_short_rows_beside_residuals_without_a_root(cuda_available, m
         listed = np.isin(gi, [100, 777]).sum(axis=1)
         assert np.all((listed == 0) | (listed == 2))
         assert np.count_nonzero(listed == 2) == idx.last_stats["overflow_queries"]
+
+
+@pytest.mark.parametrize("n,d,m,kt,k,nq", [(6001, 2, 512, 0, 20, 3000), (20001, 1, 32, 0, 1, 6000), (6001, 2, 800, 1, 7, 3000)])
+def test_digit_pass_against_the_general_kernels_of_the_same_call(cuda_available, monkeypatch, n, d, m, kt, k, nq):
+    """One call on both passes: a last row with p = NaN, which no query below it sees, sends the second index's
+    calls to the general kernels.  Every p is tiny here, where those evaluate each candidate exactly and the
+    digit pass only its survivors, which shows which of the two ran."""
+    from covertreex_gb300.device import CudaResidualIndex
+
+    case = gaussian_case(n, d, m, kt, 2.0, seed=5)
+    monkeypatch.setenv("CT_SCREEN_SURVIVOR_CAP", "64")
+    q = np.random.default_rng(6).choice(np.arange(1024, n - 1), nq, replace=False).astype(np.int64)
+    p = case["p"].copy()
+    p[n - 1] = np.nan
+    rows, share = [], []
+    for pp in (case["p"], p):
+        idx = CudaResidualIndex(case["V"], pp, case["X"], variance=1.0, lengthscale=case["ls"], kernel_type=kt,
+                                build_tree=False)
+        rows.append(idx.knn(q, k, predecessor=True, form="screened"))
+        share.append(idx.last_stats["pairs_rescored"] / idx.last_stats["pairs_exhaustive"])
+    assert share[0] < 0.5 and share[1] > 0.9, share
+    assert np.array_equal(rows[0][0], rows[1][0])
+    assert np.array_equal(rows[0][1].view(np.uint32), rows[1][1].view(np.uint32))
