@@ -983,9 +983,10 @@ struct RescoreParams {
     // survivors do not fit (set to 1, left to the exhaustive kernels)
     const int* row_query;
     int* row_bad;
-    // survivor pass: slots with more survivors than the first kernel's buffer (filled by it), count
-    int* big_list;
-    int* big_cnt;
+    // survivor pass: the slots to take (collect_overflow_kernel's big_list) instead of all, and their number
+    const int* big_list;
+    const int* big_cnt;
+    int big_blocks;
 };
 
 // ---------------------------------------------------------- double-float
@@ -1339,10 +1340,13 @@ __device__ __forceinline__ void pair_bounds_f32(const RescoreParams& P, int q, i
 //     by the double-float error of the exact distances, bounds the k-th distance.
 //  E: only survivors with dl2 <= tau are rescored exactly (compensated FP32 dot,
 //     double-float distance); the others cannot enter the top k.
-// One slot's work is a chain of short gathers, so the pass is bound by the warps in flight: a first kernel
-// with buffers of RSMALL survivors and a slice of m / 32 registers (24 warps per SM for m <= 512, not 16)
-// lists the few slots that need more for a second one.  n = 32768, m = 256: 1.72 ms -> 0.90 and 0.3;
-// n = 262144, m = 512: 15.5 -> 13.6 ms.
+// One slot's work is a chain of short gathers, so a call of many slots is bound by the warps in flight: buffers
+// of RSMALL survivors and a slice of m / 32 registers hold 24 warps per SM for m <= 512, the full buffers 16.
+// Slots with more survivors are listed beforehand for a kernel of their own, which runs beside the first one:
+// a single such slot takes 0.3 to 0.8 ms, which behind the first kernel made calls of fewer than some 20000
+// slots slower than one kernel with full buffers (n = 16384, m = 128, 2000 queries, k = 1: 0.49 ms as one
+// kernel, 0.17 and then 0.42).  Calls of one wave of the full buffers, and m > 512, take one kernel.
+// n = 32768, m = 256: 1.72 ms as one kernel, 1.1 as two.
 // Streaming top-k of E through a sorted shared buffer: entries [0, k) hold the current
 // best, new candidates fill the rest, and a full buffer is re-sorted.  Shared memory per
 // warp: BUF keys, then BUF floats (du2, reused for the kept ids).
@@ -1354,15 +1358,23 @@ __global__ void __launch_bounds__(256, PER <= 16 && BUF < RBUF ? 3 : 2) rescore_
     unsigned long long* keys = rkeys_all + (size_t)warp * BUF;
     float* du2s = (float*)(rkeys_all + (size_t)wpb * BUF) + (size_t)warp * BUF;
     int* kept = (int*)du2s;
-    // second kernel of the survivor pass: the listed slots; else all (one per warp)
+    // the listed slots, few of them spread over P.big_blocks blocks, many packed; else all, in order
     const bool listed = BUF == RBUF && P.big_list;
     const long long nw = listed ? *P.big_cnt : P.nslots;
-    for (long long w = (long long)blockIdx.x * wpb + warp; w < nw; w += (long long)gridDim.x * wpb) {
+    long long w = (long long)blockIdx.x * wpb + warp, step = (long long)gridDim.x * wpb;
+    if (listed) {
+        const long long nb = min((long long)gridDim.x, max((long long)P.big_blocks, (nw + wpb - 1) / wpb));
+        if (blockIdx.x >= nb) return;
+        w = warp * nb + blockIdx.x;
+        step = nb * wpb;
+    }
+    for (; w < nw; w += step) {
     const int slot = listed    ? P.big_list[w]
                      : P.order ? P.order[w / P.parts] * P.parts + (int)(w % P.parts)
                                : (int)w;
     const int c0 = P.surv_cnt[2 * slot];
     const int c1 = P.surv_cnt[2 * slot + 1];
+    if (BUF < RBUF && c0 + c1 > BUF) continue;  // a listed slot, or an overflowed one
     if (c0 > P.half_cap || c1 > P.half_cap) {  // handled by the exhaustive pass
         if (P.row_bad && lane == 0) P.row_bad[slot] = 1;
         continue;
@@ -1401,12 +1413,8 @@ __global__ void __launch_bounds__(256, PER <= 16 && BUF < RBUF ? 3 : 2) rescore_
             }
             const unsigned mk = __ballot_sync(0xffffffffu, keep);
             if (count + __popc(mk) > BUF) {  // (only digit rows exceed RBUF)
-                if (lane == 0) {
-                    if (BUF == RBUF) P.row_bad[slot] = 1;
-                    else P.big_list[atomicAdd(P.big_cnt, 1)] = slot;
-                }
-                fits = false;
-                break;
+                if (lane == 0) P.row_bad[slot] = 1;
+                continue;
             }
             if (keep) keys[count + __popc(mk & ((1u << lane) - 1u))] = (unsigned long long)(unsigned)cid;
             count += __popc(mk);
@@ -1572,22 +1580,23 @@ __global__ void digit_unfit_kernel(const float* __restrict__ xs, int d, const fl
     if (r < n && !digit_fit(xs, d, vn, isp, r)) atomicAdd(unfit, 1);
 }
 
-// Slots whose survivor lists overflowed; bit 31 marks those for the filtered pass.  counts: the slots listed,
-// (the survivor pass's), those whose query does not fit the digit pass.
-__global__ void collect_overflow_kernel(const int* __restrict__ surv_cnt, long long nslots, int half_cap,
-                                        const int* __restrict__ slot_id, const float* __restrict__ xs, int d,
-                                        const float* __restrict__ isp, const float* __restrict__ vn, int filter,
-                                        int* __restrict__ list, int* __restrict__ counts) {
-    long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (s >= nslots) return;
-    if (surv_cnt[2 * s] > half_cap || surv_cnt[2 * s + 1] > half_cap) {
-        const int q = slot_id[s];
-        const bool f = filter && q >= 0 && isp[q] * vn[q] <= kFilterIsq;
+// Slots whose survivor lists overflowed (bit 31 marks those for the filtered pass), and into big_list those
+// with more survivors than the survivor pass's small buffers hold.  counts: the slots of either list, the
+// overflowed slots whose query does not fit the digit pass.
+__global__ void collect_overflow_kernel(RescoreParams P, int filter, int* __restrict__ list, int* __restrict__ big_list,
+                                        int* __restrict__ counts) {
+    const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (s >= P.nslots) return;
+    const int c0 = P.surv_cnt[2 * s], c1 = P.surv_cnt[2 * s + 1];
+    if (c0 > P.half_cap || c1 > P.half_cap) {
+        const int q = P.slot_id[s];
+        const bool f = filter && q >= 0 && P.isp[q] * P.vn[q] <= kFilterIsq;
         list[atomicAdd(&counts[0], 1)] = (int)s | (f ? (int)0x80000000u : 0);
-        if (q >= 0 && !digit_fit(xs, d, vn, isp, q)) atomicAdd(&counts[2], 1);
+        if (q >= 0 && !digit_fit(P.xs, P.d, P.vn, P.isp, q)) atomicAdd(&counts[2], 1);
+    } else if (c0 + c1 > RSMALL) {
+        big_list[atomicAdd(&counts[1], 1)] = (int)s;
     }
 }
-
 
 }  // namespace screen
 }  // namespace ct
@@ -3171,34 +3180,55 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const size_t fsmem8 = filter_smem_bytes(m, 8), fsmem4 = filter_smem_bytes(m, 4);
     const bool can_filter = m <= 1024 && fsmem8 <= (size_t)smem_optin;
-    const RescoreFn surv_fn = rescore_fn(m, true), big_fn = rescore_fn(m, false);  // survivor pass
+    // Survivor pass: small buffers beside the listed slots where the slots are more than one wave of the full
+    // ones, else one kernel (two_surv)
+    const bool two_surv = m <= 512 && nslots > 16LL * sms;
+    const RescoreFn surv_fn = rescore_fn(m, true), big_fn = rescore_fn(m, false);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(surv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rescore_smem(RSMALL));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(big_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rescore_smem(RBUF));
-    R.big_list = big_list; R.big_cnt = nfull_d + 1;
     // The overflow list first: the exhaustive pass is planned on the host and runs on side
     // streams while the survivor pass runs on the call's stream.
-    int nfull = 0, unfit = 0, status = 0;
+    int counts[3] = {0, 0, 0}, status = 0;  // see collect_overflow_kernel
     long long exh_pairs = 0;  // candidates of the exhaustive pass (part tiles count whole tiles)
     cudaEvent_t ev_ovf = nullptr;
     if (e == cudaSuccess) {
-        collect_overflow_kernel<<<grid_for(nslots), 256, 0, st>>>(surv_cnt, nslots, half_cap, slot_id_use, xs, d, S->isp,
-                                                                    S->vn, can_filter ? 1 : 0, full_list, nfull_d);
+        collect_overflow_kernel<<<grid_for(nslots), 256, 0, st>>>(R, can_filter ? 1 : 0, full_list, big_list, nfull_d);
         e = cudaGetLastError();
         ++launches;
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&nfull, nfull_d, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&unfit, nfull_d + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(counts, nfull_d, sizeof(counts), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&status, S->status, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_ovf, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventRecord(ev_ovf, st);
-    if (e == cudaSuccess) {
-        const unsigned sblocks = (unsigned)((nslots + rwpb - 1) / rwpb);
-        surv_fn<<<sblocks, 32 * rwpb, rescore_smem(RSMALL), st>>>(R);
-        big_fn<<<std::min(sblocks, 2u * sms), 32 * rwpb, rescore_smem(RBUF), st>>>(R);
+    // side streams: one level above the call's.  The survivor pass fills the chip with short blocks, and a pass
+    // that started behind it would run after it (vecchia 32768 / 256: 6.57 ms, with priority 5.84)
+    int prio = 0, least = 0, greatest = 0;
+    if (e == cudaSuccess) e = cudaStreamGetPriority(st, &prio);
+    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    prio = ct::side_stream_priority(prio, greatest);
+    cudaStream_t big_st = nullptr;
+    cudaEvent_t ev_big = nullptr;
+    const unsigned sblocks = (unsigned)((nslots + rwpb - 1) / rwpb);
+    if (two_surv) {  // the listed slots first (see rescore_kernel)
+        RescoreParams B = R;
+        B.big_list = big_list; B.big_cnt = nfull_d + 1; B.big_blocks = 2 * sms;
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&big_st, cudaStreamNonBlocking, prio);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_big, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(big_st, ev_ovf, 0);
+        if (e == cudaSuccess) {
+            big_fn<<<std::min(sblocks, 16u * sms), 32 * rwpb, rescore_smem(RBUF), big_st>>>(B);
+            surv_fn<<<sblocks, 32 * rwpb, rescore_smem(RSMALL), st>>>(R);
+            e = cudaGetLastError();
+            launches += 2;
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(ev_big, big_st);
+    } else if (e == cudaSuccess) {
+        big_fn<<<sblocks, 32 * rwpb, rescore_smem(RBUF), st>>>(R);
         e = cudaGetLastError();
-        launches += 2;
+        ++launches;
     }
     if (e == cudaSuccess) e = cudaEventSynchronize(ev_ovf);
+    const int nfull = counts[0], unfit = counts[2];
     ExhGroup* groups_d = nullptr;
     ExhItem* xitems_d = nullptr;
     int* item_begin_d = nullptr;
@@ -3208,12 +3238,6 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     DigitRun digits;
     int nexh = nfull;  // slots left to the exhaustive kernels
     if (e == cudaSuccess && nfull > 0) {
-        // one level above the call's stream: the survivor pass fills the chip with short blocks, and a pass that
-        // started behind it would run after it (vecchia 32768 / 256: 6.57 ms, with priority 5.84)
-        int prio = 0, least = 0, greatest = 0;
-        e = cudaStreamGetPriority(st, &prio);
-        if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
-        prio = ct::side_stream_priority(prio, greatest);
         for (auto& a : aux)
             if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&a, cudaStreamNonBlocking, prio);
         for (auto& v : ev_aux)
@@ -3443,6 +3467,12 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     for (auto& v : ev_aux)
         if (v) cudaEventDestroy(v);
     if (ev_ovf) cudaEventDestroy(ev_ovf);
+    if (big_st) {  // the call's stream goes on, and frees, after the listed slots
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_big, 0);
+        if (e != cudaSuccess) cudaStreamSynchronize(big_st);
+        cudaStreamDestroy(big_st);
+    }
+    if (ev_big) cudaEventDestroy(ev_big);
     if (e == cudaSuccess && parts > 1) {
         merge_parts_kernel<<<(unsigned)((nq + 7) / 8), 256, 0, st>>>(part_idx, part_dist, nq, parts, k,
                                                                      (long long*)out_idx, out_dist);

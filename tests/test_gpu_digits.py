@@ -160,3 +160,21 @@ def test_digit_pass_against_the_general_kernels_of_the_same_call(cuda_available,
     assert share[0] < 0.5 and share[1] > 0.9, share
     assert np.array_equal(rows[0][0], rows[1][0])
     assert np.array_equal(rows[0][1].view(np.uint32), rows[1][1].view(np.uint32))
+
+
+@pytest.mark.parametrize("m,k,nq", [(512, 64, 700), (512, 1, 700), (544, 64, 700), (96, 50, 3000)])
+@pytest.mark.parametrize("predecessor", [False, True])
+def test_survivor_pass_with_listed_slots(cuda_available, m, k, nq, predecessor):
+    """More slots than one wave of full buffers: those with over 512 survivors are listed for a kernel of their
+    own (at m = 544 none, one kernel takes all); calls of 40 queries are one kernel throughout."""
+    from covertreex_gb300.device import CudaResidualIndex
+
+    case = mixture_case(16384, 8, m, 2.0)
+    idx = CudaResidualIndex(case["V"], case["p"], case["X"], variance=1.0, lengthscale=case["ls"], kernel_type=0,
+                            build_tree=False)
+    q = np.random.default_rng(8).choice(16384, nq, replace=False).astype(np.int64)
+    gi, gd = idx.knn(q, k, predecessor=predecessor, form="screened")
+    for s in range(0, 400, 40):
+        hi, hd = idx.knn(q[s:s + 40], k, predecessor=predecessor, form="screened")
+        assert np.array_equal(hi, gi[s:s + 40])
+        assert np.array_equal(hd.view(np.uint32), gd[s:s + 40].view(np.uint32))
