@@ -3200,19 +3200,21 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     if (e == cudaSuccess) e = cudaMemcpyAsync(&status, S->status, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_ovf, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventRecord(ev_ovf, st);
-    // side streams: one level above the call's.  The survivor pass fills the chip with short blocks, and a pass
-    // that started behind it would run after it (vecchia 32768 / 256: 6.57 ms, with priority 5.84)
+    // The listed slots and the digit pass run one level above the call's stream: the survivor pass fills the chip
+    // with short blocks, and a pass that started behind it would run after it (vecchia 32768 / 256: 6.57 ms, with
+    // priority 5.84).  The general exhaustive kernels keep the call's level: ahead of the survivor pass they
+    // hold the SMs that its long slots need (n = 3000, m = 1024, predecessors: 5.2 ms, 4.3 beside it).
     int prio = 0, least = 0, greatest = 0;
     if (e == cudaSuccess) e = cudaStreamGetPriority(st, &prio);
     if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
-    prio = ct::side_stream_priority(prio, greatest);
+    const int side = ct::side_stream_priority(prio, greatest);
     cudaStream_t big_st = nullptr;
     cudaEvent_t ev_big = nullptr;
     const unsigned sblocks = (unsigned)((nslots + rwpb - 1) / rwpb);
     if (two_surv) {  // the listed slots first (see rescore_kernel)
         RescoreParams B = R;
         B.big_list = big_list; B.big_cnt = nfull_d + 1; B.big_blocks = 2 * sms;
-        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&big_st, cudaStreamNonBlocking, prio);
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&big_st, cudaStreamNonBlocking, side);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_big, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(big_st, ev_ovf, 0);
         if (e == cudaSuccess) {
@@ -3281,7 +3283,13 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
                 for (auto& x : uq) std::swap(x.first, x.second);
                 std::vector<int> bad;
                 int dstatus = 0;
-                e = digit_pass(R, S->vn_max, qtau, n, uq, sms, x0, &digits, &bad, &dstatus, &launches);
+                cudaStream_t xd = nullptr;
+                e = cudaStreamCreateWithPriority(&xd, cudaStreamNonBlocking, side);
+                if (e == cudaSuccess) {  // (the overflow list's copies above have passed ev_ovf)
+                    e = digit_pass(R, S->vn_max, qtau, n, uq, sms, xd, &digits, &bad, &dstatus, &launches);
+                    cudaStreamSynchronize(xd);  // its results are read, and freed, on the call's stream
+                    cudaStreamDestroy(xd);
+                }
                 if (dstatus != 0) status = dstatus;
                 if (e == cudaErrorMemoryAllocation) {  // no room: the kernels below need little
                     cudaGetLastError();
