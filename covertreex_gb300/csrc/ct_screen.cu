@@ -3234,16 +3234,12 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
     ExhItem* xitems_d = nullptr;
     int* item_begin_d = nullptr;
     unsigned long long* partial = nullptr;
-    cudaStream_t aux[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t ev_aux[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    cudaStream_t x0 = nullptr, aux[4] = {nullptr, nullptr, nullptr, nullptr};  // plan and digit pass; general kernels
+    cudaEvent_t ev_aux[4] = {nullptr, nullptr, nullptr, nullptr};
     DigitRun digits;
     int nexh = nfull;  // slots left to the exhaustive kernels
     if (e == cudaSuccess && nfull > 0) {
-        for (auto& a : aux)
-            if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&a, cudaStreamNonBlocking, prio);
-        for (auto& v : ev_aux)
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
-        cudaStream_t x0 = aux[0];
+        e = cudaStreamCreateWithPriority(&x0, cudaStreamNonBlocking, side);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(x0, ev_ovf, 0);
         auto AX = [&](void** ptr, size_t bytes) { if (e == cudaSuccess) e = cudaMallocAsync(ptr, bytes ? bytes : 16, x0); };
         // Group the overflowed slots that share a candidate source and split each group's
@@ -3282,13 +3278,7 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
                 for (auto& x : uq) std::swap(x.first, x.second);
                 std::vector<int> bad;
                 int dstatus = 0;
-                cudaStream_t xd = nullptr;
-                e = cudaStreamCreateWithPriority(&xd, cudaStreamNonBlocking, side);
-                if (e == cudaSuccess) {  // (the overflow list's copies above have passed ev_ovf)
-                    e = digit_pass(R, S->vn_max, qtau, n, uq, sms, xd, &digits, &bad, &dstatus, &launches);
-                    cudaStreamSynchronize(xd);  // its results are read, and freed, on the call's stream
-                    cudaStreamDestroy(xd);
-                }
+                e = digit_pass(R, S->vn_max, qtau, n, uq, sms, x0, &digits, &bad, &dstatus, &launches);
                 if (dstatus != 0) status = dstatus;
                 if (e == cudaErrorMemoryAllocation) {  // no room: the kernels below need little
                     cudaGetLastError();
@@ -3425,50 +3415,61 @@ int ct_tree::knn_screened(const int64_t* q_ids, int64_t nq, int k, int predecess
         if (e == cudaSuccess && koff[3] > koff[2])
             e = cudaFuncSetAttribute(filter_tile_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem4);
         if (e == cudaSuccess && nitems > 0) {
-            // the kinds run side by side; merge_chunks waits for all three
-            if (koff[1] > koff[0]) {
-                tile_fn<<<(unsigned)(koff[1] - koff[0]), 256, tsmem, x0>>>(
+            // the kinds run side by side, each on a stream of its own; merge_chunks waits for all
+            int main = -1;
+            for (int kd = 0; kd < 4; ++kd) {
+                if (koff[kd + 1] == koff[kd]) continue;
+                if (main < 0) main = kd;
+                if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&aux[kd], cudaStreamNonBlocking, prio);
+                if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_aux[kd], cudaEventDisableTiming);
+            }
+            if (e == cudaSuccess && koff[1] > koff[0]) {
+                tile_fn<<<(unsigned)(koff[1] - koff[0]), 256, tsmem, aux[0]>>>(
                     R, groups_d, xitems_d + koff[0], item_begin_d, kchunk[0], ktpc[0], units_d, S->lvl_id, S->b_id_ds,
                     partial);
                 ++launches;
             }
-            if (koff[2] > koff[1]) {
+            if (e == cudaSuccess && koff[2] > koff[1]) {
                 filter_tile_kernel<8><<<(unsigned)(koff[2] - koff[1]), 256, fsmem8, aux[1]>>>(
                     R, groups_d, xitems_d + koff[1], item_begin_d, kchunk[1], ktpc[1], units_d, S->lvl_id, S->b_id_ds,
                     partial);
                 ++launches;
             }
-            if (koff[3] > koff[2]) {
+            if (e == cudaSuccess && koff[3] > koff[2]) {
                 filter_tile_kernel<4><<<(unsigned)(koff[3] - koff[2]), 256, fsmem4, aux[2]>>>(
                     R, groups_d, xitems_d + koff[2], item_begin_d, kchunk[2], ktpc[2], units_d, S->lvl_id, S->b_id_ds,
                     partial);
                 ++launches;
             }
-            if (koff[4] > koff[3]) {
+            if (e == cudaSuccess && koff[4] > koff[3]) {
                 const int nw = koff[4] - koff[3];
                 rescore_warp_kernel<<<(unsigned)((nw + 7) / 8), 256, 0, aux[3]>>>(
                     R, groups_d, xitems_d + koff[3], nw, item_begin_d, kchunk[3], ktpc[3], units_d, S->lvl_id,
                     S->b_id_ds, partial);
                 ++launches;
             }
-            e = cudaGetLastError();
-            for (int a = 1; a < 4; ++a) {
-                if (e == cudaSuccess) e = cudaEventRecord(ev_aux[a], aux[a]);
-                if (e == cudaSuccess) e = cudaStreamWaitEvent(x0, ev_aux[a], 0);
+            if (e == cudaSuccess) e = cudaGetLastError();
+            for (int kd = main + 1; kd < 4; ++kd) {
+                if (!aux[kd]) continue;
+                if (e == cudaSuccess) e = cudaEventRecord(ev_aux[kd], aux[kd]);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(aux[main], ev_aux[kd], 0);
             }
             if (e == cudaSuccess) {
-                merge_chunks_kernel<<<(unsigned)((nexh + rwpb - 1) / rwpb), 32 * rwpb, rsmem, x0>>>(R, item_begin_d, partial);
+                merge_chunks_kernel<<<(unsigned)((nexh + rwpb - 1) / rwpb), 32 * rwpb, rsmem, aux[main]>>>(R, item_begin_d, partial);
                 e = cudaGetLastError();
                 ++launches;
             }
+            if (e == cudaSuccess) e = cudaEventRecord(ev_aux[main], aux[main]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_aux[main], 0);
         }
         }
-        if (e == cudaSuccess) e = cudaEventRecord(ev_aux[4], x0);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_aux[4], 0);
-        if (e != cudaSuccess)  // nothing of the side streams may outlive the buffers freed below
+        if (e != cudaSuccess) {  // nothing of the side streams may outlive the buffers freed below
+            if (x0) cudaStreamSynchronize(x0);
             for (auto& a : aux)
                 if (a) cudaStreamSynchronize(a);
+        }
     }
+    if (x0) cudaStreamDestroy(x0);  // (the host has waited for its work)
     for (auto& a : aux)
         if (a) cudaStreamDestroy(a);
     for (auto& v : ev_aux)
