@@ -24,12 +24,16 @@
 // the lists through distributed shared memory (no scratch, no second launch), more of them go
 // through scratch and a counter.
 //
+// Few points (some 600 at most) and few queries take a warp per query instead: the tile's fixed chain
+// (thresholds, then four queries' sorts per warp) is 6 to 12 us there against 1 to 3.
+//
 // Measured on GB300 (whole calls, queries = the points; before: a warp per query with a sorted list
 // of k per lane, so that a warp ran k insertion steps for every point any lane took):
 //   n = 32768, d = 3, k = 10     4.49 -> 0.71 ms (9.0 T lane operations/s of 39 measured; without
 //                                the sampled thresholds 1.11 ms)
 //   n = 65536, d = 3, k = 10    14.8  -> 2.30 ms;   n = 65536, d = 8, k = 50, predecessors 54.1 -> 3.3 ms
 //   n = 1024,  d = 3, k = 10    23 us both (the host's share of a call)
+//   n = 50,    d = 3, k = 10    16.5 us, 22.5 with the tile
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -374,6 +378,102 @@ __global__ void __launch_bounds__(kEThreads, 2) euclid_knn_kernel(EParams P) {
     }
 }
 
+// The form for few points: one warp per query, eight queries per block.  Points are staged through shared
+// memory; lane l scores points l, l + 32, ... and keeps its own K best (d^2, index) in registers, sorted (a
+// lane sees its points in increasing index, so a tie keeps the lower index).  The warp merges its 32 lists
+// with k rounds of a warp-wide (d^2, index) minimum.
+constexpr int kSTile = 512;
+
+__device__ __forceinline__ bool dl_less(float da, int ia, float db, int ib) {
+    return da < db || (da == db && ia < ib);
+}
+
+template <int K>
+__global__ void __launch_bounds__(kEThreads) euclid_small_kernel(EParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* tile = (float*)smem_raw;  // kSTile * d floats
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, d = P.d;
+    const long long qi = (long long)blockIdx.x * kEWarps + warp;
+    const bool active = qi < P.nq;
+    float q[kEMaxD];
+#pragma unroll
+    for (int c = 0; c < kEMaxD; ++c) q[c] = (active && c < d) ? P.qry[qi * d + c] : 0.f;
+    float bd[K];
+    int bi[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) { bd[j] = CT_FLT_MAX; bi[j] = 0x7fffffff; }
+    const long long limit = P.predecessor ? (active ? qi : 0) : P.n;
+    // the block needs points below the largest limit of its queries
+    const long long block_limit = P.predecessor ? min(P.n, ((long long)blockIdx.x + 1) * kEWarps) : P.n;
+    for (long long t0 = 0; t0 < block_limit; t0 += kSTile) {
+        const int tn = (int)min((long long)kSTile, block_limit - t0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < tn * d; e += kEThreads) tile[e] = P.pts[t0 * d + e];
+        __syncthreads();
+        if (!active) continue;
+        const int jn = (int)min((long long)tn, limit - t0);
+        for (int j = lane; j < jn; j += 32) {
+            float s = 0.f;
+            for (int c = 0; c < d; ++c) {
+                const float df = __fsub_rn(q[c], tile[j * d + c]);
+                s = __fmaf_rn(df, df, s);
+            }
+            if (s < bd[K - 1]) {  // strict: an equal distance seen later has a larger index
+                const int gj = (int)(t0 + j);
+#pragma unroll
+                for (int p = K - 1; p > 0; --p) {
+                    const bool up = s < bd[p - 1];
+                    const bool here = !up && s < bd[p];
+                    bd[p] = up ? bd[p - 1] : (here ? s : bd[p]);
+                    bi[p] = up ? bi[p - 1] : (here ? gj : bi[p]);
+                }
+                if (s < bd[0]) { bd[0] = s; bi[0] = gj; }
+            }
+        }
+    }
+    if (!active) return;
+    int head = 0;
+    for (int r = 0; r < P.k; ++r) {
+        float hd = CT_FLT_MAX;
+        int hi = 0x7fffffff;
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (j == head) { hd = bd[j]; hi = bi[j]; }
+        float md = hd;
+        int mi = hi;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const float od = __shfl_xor_sync(0xffffffffu, md, off);
+            const int oi = __shfl_xor_sync(0xffffffffu, mi, off);
+            if (dl_less(od, oi, md, mi)) { md = od; mi = oi; }
+        }
+        if (hd == md && hi == mi && hi != 0x7fffffff) ++head;
+        if (lane == 0) {
+            const bool ok = mi != 0x7fffffff && md < CT_FLT_MAX;
+            P.out_idx[qi * P.k + r] = ok ? (long long)mi : -1LL;
+            P.out_dist[qi * P.k + r] = ok ? sqrtf(md) : CT_FLT_MAX;
+        }
+    }
+}
+
+// Where it is the faster form (n = 16 to 1500, 1 to 40000 queries, k = 1 to 24, d = 1 to 16, both timed): up
+// to 600 - 8 k points (n = 400, 300 queries, d = 3: k = 1 15 against 19 us, k = 24 28 against 32; n = 700,
+// k = 16 even), while one wave of warps takes the queries; and with eight queries at most, one per warp of
+// the tile, for the shortest lists or more than 8 axes only.  A predecessor search sees no more points than
+// it has queries.
+bool small_form(long long n, long long nq, int d, int k, int predecessor) {
+    if (predecessor) n = std::min(n, nq);
+    return n + 8 * k <= 600 && k <= (nq > 8 || d > 8 ? 24 : 4) &&
+           (double)nq * (double)n * k <= (nq <= 1000 ? 3e6 : 2e6);
+}
+
+template <int K>
+cudaError_t launch_small(const EParams& P, cudaStream_t st) {
+    const size_t smem = sizeof(float) * kSTile * (size_t)P.d;  // at most 32 KB
+    euclid_small_kernel<K><<<(unsigned)((P.nq + kEWarps - 1) / kEWarps), kEThreads, smem, st>>>(P);
+    return cudaGetLastError();
+}
+
 // Sampled steps of a chunk of L points: a sample of M points leaves about 1.2 k L / M points under
 // the threshold, each worth some 480 pairs of distances (its warp's detour and its share of a
 // merge) at d = 3, fewer where a pair costs more (about 2 d + 2 instructions), so M grows as
@@ -428,6 +528,12 @@ cudaError_t launch_d(const EParams& P, long long items, cudaStream_t st) {
 cudaError_t launch_euclid_knn(const float* pts, long long n, int d, const float* qry, long long nq, int k,
                               int predecessor, long long* out_idx, float* out_dist, cudaStream_t st) {
     if (nq <= 0) return cudaSuccess;
+    if (small_form(n, nq, d, k, predecessor)) {
+        EParams S{};
+        S.pts = pts; S.qry = qry; S.n = n; S.nq = nq; S.d = d; S.k = k; S.predecessor = predecessor;
+        S.out_idx = out_idx; S.out_dist = out_dist;
+        return k <= 16 ? launch_small<16>(S, st) : launch_small<32>(S, st);
+    }
     int dev = 0, sms = 148;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -78,3 +78,20 @@ def test_infinite_and_nan_points_are_no_neighbours(cuda_available):
     P[5], P[6, 1], P[7, 2] = np.nan, np.inf, 3e38
     gi, _ = EuclideanTree(P).knn_device(P[:4], 64)
     assert not np.isin(gi.cpu().numpy(), [5, 6, 7]).any()
+
+
+@pytest.mark.parametrize("n,nq,k", [(592, 40, 1), (593, 40, 1), (472, 9, 16), (473, 9, 16), (568, 8, 4), (560, 8, 5),
+                                    (408, 33, 24), (409, 33, 24), (400, 12, 17), (512, 390, 10), (512, 400, 10),
+                                    (16, 20000, 4), (300, 20000, 10)])
+@pytest.mark.parametrize("d", [1, 3, 16])
+def test_few_points_on_both_sides_of_the_line(cuda_available, n, nq, k, d):
+    """The warp-per-query form and the tile around the line between them, with repeated points (ties by index)
+    and points that are no neighbours."""
+    r = np.random.default_rng(n + nq + k + d)
+    P = r.standard_normal((n, d)).astype(np.float32)
+    P[n // 2:n // 2 + 8] = P[:8]
+    Q = P[r.integers(0, n, nq)] if nq <= n else r.standard_normal((nq, d)).astype(np.float32)
+    _check(P, Q, k, False)
+    _check(P, P[:min(n, nq)], k, True)
+    P[5], P[n - 3] = np.nan, np.inf
+    _check(P, Q, k, False)
