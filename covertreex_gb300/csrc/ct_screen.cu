@@ -2578,12 +2578,12 @@ struct DigitRun {
 };
 // Estimated microseconds of both exhaustive passes for nslots overflowed slots: the general kernels at
 // 3e-7 per pair and column of V for slots that their FP32 filter serves and 6e-7 for the others, after a
-// latency that grows with the slots (they run beside the survivor pass, which hides most of it); the digit
+// latency that grows with the slots (they run beside the survivor pass, which hides much of it); the digit
 // pass at 4.3e-8 after 200 us and the split of the dataset.  Fitted on 464 calls with overflowed slots, n =
 // 8192 to 131072, m = 64 to 512, with either pass forced: the choice costs 0.6% of the faster one on average,
-// 15 calls lose more than 5% (general everywhere costs 94%, digits everywhere 4%).
+// 12 calls lose more than 5% (general everywhere costs 94%, digits everywhere 4%).
 static bool digits_pay(int m, int nslots, double filtered, double plain, double total, long long rows) {
-    return std::min(150.0, 3.0 * nslots) + m * (3e-7 * filtered + 6e-7 * plain) >
+    return std::min(185.0, 3.0 * nslots) + m * (3e-7 * filtered + 6e-7 * plain) >
            200.0 + 5e-6 * (double)rows * m + 4.3e-8 * m * total;
 }
 constexpr size_t kDigitSlabBytes = size_t(4) << 30;
