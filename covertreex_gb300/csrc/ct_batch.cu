@@ -67,8 +67,8 @@ constexpr size_t kHeaderBytes = 64;
 constexpr int kMaxSplit = 128;
 
 // One launch serves problems of every tile height: each problem carries its own configuration.
-// NT = 256: the forms that run two blocks per SM; NT = 512: the forms for wide rows, when a
-// problem of the batch fits no other.
+// NT = 256: the forms that run two blocks per SM (one, where a problem's rows are too wide for
+// half of one); NT = 512: the forms that take an SM with 16 warps (launch_mode chooses).
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     batch_kernel(const unsigned char* __restrict__ desc, unsigned long long* __restrict__ ctr, dense::u64 nz) {
@@ -252,34 +252,58 @@ struct Config {
     dense::Ring ring{};
     size_t smem = 0;
 };
-bool config_for(const ct_batch* B, int m, int d, int k, long long nq, int qt, bool wide, Config* c) {
-    const int tall = wide ? dense::kCfg32w : dense::kCfg32, low = wide ? dense::kCfg16w : dense::kCfg16;
-    const size_t limit = dense::cfg_limit(tall, B->smem_optin, B->smem_per_sm, kStaticSmem);
+// Launches: two blocks of 256 threads per SM, one of them (for wider rows), one of 512 threads.
+enum Mode { kTwo = 0, kOne = 1, kWide = 2, kNoMode = -1 };
+bool config_for(const ct_batch* B, int m, int d, int k, long long nq, int qt, int mode, Config* c) {
+    const int tall = mode == kWide ? dense::kCfg32w : dense::kCfg32, low = mode == kWide ? dense::kCfg16w : dense::kCfg16;
+    const size_t limit = mode == kTwo ? dense::cfg_limit(tall, B->smem_optin, B->smem_per_sm, kStaticSmem)
+                                      : B->smem_optin - kStaticSmem;
     c->cfg = tall;
     if (qt != 16 && (qt != 0 || nq > 16) && dense::pick_ring(tall, m, d, k, limit, &c->ring, &c->smem)) return true;
     c->cfg = low;
     return dense::pick_ring(low, m, d, k, limit, &c->ring, &c->smem);
 }
 
-bool all_fit(const ct_batch* B, bool wide) {
-    Config c;
-    if (!config_for(B, B->res_m, B->res_d, B->res_k, 1, 0, wide, &c)) return false;
-    for (const BatchReq& r : B->reqs)
-        if (!config_for(B, r.tree->m, r.tree->d, r.k, r.nq, 0, wide, &c)) return false;
-    return true;
+// The launch that takes the batch's pairs in the least estimated time, each problem in its own tile height;
+// kNoMode when none holds every problem and the reserved sizes.  Two blocks per SM, in 16-row tiles if need be,
+// unless their stages are narrow (m > 512): there a block per SM in 32-row tiles is 1.1 to 1.15 times as fast
+// (two sets of 700 to 4096 queries against n = 4096, m = 1024), at m = 256 and k = 60 it is 4% slower.
+int launch_mode(const ct_batch* B, int qt) {
+    const double tall_cost[3] = {1.0, 1.3, 1.26};
+    int best = kNoMode;
+    double best_t = 0.0;
+    long long queries = 0;
+    for (const BatchReq& r : B->reqs) queries += r.nq;
+    for (int mode = kTwo; mode <= kWide; ++mode) {
+        // (a few queries are split finer in 16-row tiles: two sets of 40, m = 768, 1.2 times as fast)
+        if (mode == kOne && queries < 512) continue;
+        Config c;
+        bool fits = config_for(B, B->res_m, B->res_d, B->res_k, 1, 0, mode, &c);
+        double t = 0.0;
+        for (const BatchReq& r : B->reqs) {
+            fits = fits && config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, mode, &c);
+            if (!fits) break;
+            const int height = dense::cfg_qt(c.cfg);
+            const double cost = height == 32 ? tall_cost[mode] : mode == kTwo && c.ring.wmax == 64 ? 1.25 : 1.6;
+            t += (double)((r.nq + height - 1) / height * height) * (double)r.tree->n * r.tree->m * cost;
+        }
+        if (fits && (best == kNoMode || t < best_t)) {
+            best = mode;
+            best_t = t;
+        }
+    }
+    return best;
 }
-// Rows too wide for two blocks per SM take the whole batch to the 512-thread kernel.
-bool is_wide(const ct_batch* B) { return !all_fit(B, false); }
 
 // Shared memory of a launch: the largest of the batch's problems and of the reserved (m, d, k) in
 // either height.
-size_t smem_for(const ct_batch* B, int qt, bool wide) {
+size_t smem_for(const ct_batch* B, int qt, int mode) {
     size_t most = 0;
     Config c;
     for (const BatchReq& r : B->reqs)
-        if (config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, wide, &c)) most = std::max(most, c.smem);
+        if (config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, mode, &c)) most = std::max(most, c.smem);
     for (int nq = 16; nq <= 32; nq += 16)
-        if (config_for(B, B->res_m, B->res_d, B->res_k, nq, qt, wide, &c)) most = std::max(most, c.smem);
+        if (config_for(B, B->res_m, B->res_d, B->res_k, nq, qt, mode, &c)) most = std::max(most, c.smem);
     return most;
 }
 
@@ -297,7 +321,7 @@ int plan_qt(const Plan& P) {
 }
 
 // Order problems, choose each problem's candidate split and lay out its scratch.
-void make_plan(const ct_batch* B, int qt, int cps, int ips, bool wide, Plan& P) {
+void make_plan(const ct_batch* B, int qt, int cps, int ips, int mode, Plan& P) {
     const int nr = (int)B->reqs.size();
     std::vector<int> ord;
     std::vector<double> tile_work(nr, 0.0);
@@ -307,7 +331,7 @@ void make_plan(const ct_batch* B, int qt, int cps, int ips, bool wide, Plan& P) 
     for (int i = 0; i < nr; ++i) {
         const BatchReq& r = B->reqs[i];
         if (r.nq <= 0) continue;
-        config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, wide, &cfgs[i]);
+        config_for(B, r.tree->m, r.tree->d, r.k, r.nq, qt, mode, &cfgs[i]);
         const int height = dense::cfg_qt(cfgs[i].cfg);
         const long long tiles = (r.nq + height - 1) / height;
         const double per_pair = (double)r.tree->m + 4.0 * r.tree->d + 16.0;
@@ -412,9 +436,9 @@ int ensure_capacity(ct_batch* B, const Plan& P, cudaStream_t st) {
 
 int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_t st) {
     Plan P;
-    const bool wide = is_wide(B);
-    if (wide) cps = 1;
-    make_plan(B, qt, cps, ips, wide, P);
+    const int mode = launch_mode(B, qt);  // (the callers have refused kNoMode)
+    if (mode != kTwo) cps = 1;
+    make_plan(B, qt, cps, ips, mode, P);
     B->last_items = P.total_items;
     B->last_pairs = P.pairs;
     B->last_qt = qt ? qt : plan_qt(P); B->last_cps = cps; B->last_ips = ips;
@@ -441,9 +465,9 @@ int run_shape(ct_batch* B, int qt, int cps, int ips, bool use_graph, cudaStream_
     memcpy(B->h_desc + kHeaderBytes, P.probs.data(), sizeof(Problem) * P.probs.size());
     const size_t copy_bytes = kHeaderBytes + sizeof(Problem) * P.probs.size();
 
-    const size_t smem = smem_for(B, qt, wide);
-    const unsigned threads = wide ? 512 : 256;
-    KernelFn fn = kernel_for(wide);
+    const size_t smem = smem_for(B, qt, mode);
+    const unsigned threads = mode == kWide ? 512 : 256;
+    KernelFn fn = kernel_for(mode == kWide);
     cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return B->cuda_err(e, "ct_batch: shared-memory attribute");
     long long grid = (long long)B->num_sms * cps;
@@ -589,7 +613,7 @@ int ct_batch_run(ct_batch* B, int32_t use_graph, ct_stats* stats, void* stream) 
         if (r.tree->m % 16 != 0) return ct::batch_fail("ct_batch_run", "tree rank m must be a multiple of 16", CT_ERR_UNSUPPORTED);
     int qt, cps, ips;
     default_shape(B, qt, cps, ips);
-    if (is_wide(B) && !all_fit(B, true))
+    if (launch_mode(B, qt) == kNoMode)
         return ct::batch_fail("ct_batch_run", "the batch's largest m, d, k exceed shared memory", CT_ERR_UNSUPPORTED);
     cudaStream_t st = (cudaStream_t)stream;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -625,8 +649,7 @@ int ct_batch_autotune(ct_batch* B, int32_t reps, void* stream, int32_t* qt_out, 
     cudaStream_t st = (cudaStream_t)stream;
     if (reps <= 0) reps = 1;
     const Shape shapes[4] = {{32, 2}, {32, 1}, {16, 2}, {16, 1}};
-    const bool wide = is_wide(B);
-    if (wide && !all_fit(B, true))
+    if (launch_mode(B, 0) == kNoMode)
         return ct::batch_fail("ct_batch_autotune", "no launch shape fits shared memory", CT_ERR_UNSUPPORTED);
     const int ipss[3] = {1, 4, 16};
     float best = 3.4e38f;
@@ -636,11 +659,12 @@ int ct_batch_autotune(ct_batch* B, int32_t reps, void* stream, int32_t* qt_out, 
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     for (const Shape& s : shapes) {
-        if (wide && s.cps > 1) continue;
+        const int mode = launch_mode(B, s.qt);
+        if (mode == kNoMode || (mode != kTwo && s.cps > 1)) continue;
         std::vector<std::vector<int>> seen;  // split patterns already timed for this shape
         for (int ips : ipss) {
             Plan P;
-            make_plan(B, s.qt, s.cps, ips, wide, P);
+            make_plan(B, s.qt, s.cps, ips, mode, P);
             std::vector<int> splits;
             for (const Problem& pr : P.probs) { splits.push_back(pr.split); splits.push_back(pr.cfg); }
             if (std::find(seen.begin(), seen.end(), splits) != seen.end()) continue;  // same launch

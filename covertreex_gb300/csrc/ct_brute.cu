@@ -96,14 +96,19 @@ Shape choose_shape(const BruteParams& P, long long cands, const Limits& L, bool 
     Shape best;
     double best_t = 0.0;
     // time of a query-candidate pair with every block slot busy, relative to the 32-row tile
-    // (the 16-row tiles reuse each operand half as often)
-    const double pair_cost[dense::kNumCfg] = {1.0, 1.25, 1.1, 1.6};
-    for (int c = 0; c < dense::kNumCfg; ++c) {
+    // (the 16-row tiles reuse each operand half as often); the last is the 32-row tile with an SM to itself, for
+    // rows too wide for the other 32-row forms (m = 528 to 1024) and calls of enough tiles to fill the chip
+    // (4096 rows against 4096, k = 10: m = 768 1.3 times as fast as 16-row tiles, m = 1024 1.46 times)
+    const double pair_cost[dense::kNumCfg + 1] = {1.0, 1.25, 1.1, 1.6, 1.15};
+    for (int i = 0; i <= dense::kNumCfg; ++i) {
+        if (i == dense::kNumCfg && P.nq < 512) break;
+        const int c = i < dense::kNumCfg ? i : dense::kCfg32;
         Shape s;
         s.cfg = c;
-        if (!dense::pick_ring(c, P.m, P.d, P.k, dense::cfg_limit(c, L.optin, L.per_sm, kFixedSmem), &s.ring, &s.smem))
-            continue;
-        const int qt = dense::cfg_qt(c), ct = dense::cfg_ct(c), bps = dense::cfg_threads(c) == 256 ? 2 : 1;
+        const size_t limit = i < dense::kNumCfg ? dense::cfg_limit(c, L.optin, L.per_sm, kFixedSmem) : L.optin - kFixedSmem;
+        if (!dense::pick_ring(c, P.m, P.d, P.k, limit, &s.ring, &s.smem)) continue;
+        const int qt = dense::cfg_qt(c), ct = dense::cfg_ct(c);
+        const int bps = i < dense::kNumCfg && dense::cfg_threads(c) == 256 ? 2 : 1;
         const long long tiles = (P.nq + qt - 1) / qt;
         const double slots = (double)L.sms * bps;
         const int max_split =
@@ -116,7 +121,7 @@ Shape choose_shape(const BruteParams& P, long long cands, const Limits& L, bool 
             // equal items run in whole waves; predecessor tiles of falling length fill the gaps
             const double waves = P.predecessor ? std::max(items * mean / slots, len)
                                                : std::ceil(items / slots) * len;
-            const double t = waves * qt * bps * pair_cost[c] ;
+            const double t = waves * qt * bps * pair_cost[i];
             if (best.cfg < 0 || t < best_t) {
                 best = s;
                 best.split = sp;

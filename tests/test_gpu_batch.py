@@ -151,3 +151,30 @@ def test_new_points_alone_and_in_the_mix(trees):
     for (i, d), (ai, ad) in zip(mixed, alone):
         assert np.array_equal(i.cpu().numpy(), ai) and np.array_equal(d.cpu().numpy(), ad)
     _assert_exact(trees, [(i.cpu().numpy(), d.cpu().numpy()) for i, d in ids])
+
+
+@pytest.mark.parametrize("ms", [(528,), (768, 64), (1024,), (512, 1024), (1152, 256), (768, 528, 128)])
+@pytest.mark.parametrize("nq", [9, 33, 700])
+def test_launch_forms_of_wide_rows(cuda_available, ms, nq):
+    """Rows for which a block of 256 threads takes an SM alone, beside narrower ones and wider ones."""
+    from covertreex_gb300.device import CudaBatch, CudaResidualIndex
+
+    b, refs = CudaBatch(), []
+    for j, m in enumerate(ms):
+        r = np.random.default_rng(m + j)
+        n, kt = 900 + 64 * j, j % 2
+        X = r.standard_normal((n, 3)).astype(np.float32)
+        V = (r.standard_normal((n, m)) * np.sqrt(0.8 / m)).astype(np.float32)
+        p = r.uniform(1e-3, 1.0, n).astype(np.float32)
+        idx = CudaResidualIndex(V, p, X, variance=1.0, lengthscale=[1.1] * 3, kernel_type=kt, build_tree=False)
+        q = r.choice(n, nq, replace=False)
+        pred = bool(j % 2)
+        ref = O.brute_knn_f32(V, p, X, 1.0, np.full(3, 1.1, np.float32), kt, q, 20, pred)
+        refs.append((idx, b.add_ids(idx, q, 20, predecessor=pred), ref))
+        gi, gd = idx.knn(q, 20, predecessor=pred, form="dense")
+        assert np.array_equal(gi, ref[0]) and np.array_equal(gd.view(np.uint32), ref[1].view(np.uint32))
+    for _ in range(2):
+        b.run()
+        for _, (gi, gd), ref in refs:
+            assert np.array_equal(gi.cpu().numpy(), ref[0])
+            assert np.array_equal(gd.cpu().numpy().view(np.uint32), ref[1].view(np.uint32))
