@@ -1414,7 +1414,8 @@ __global__ void __launch_bounds__(256, PER <= 16 && BUF < RBUF ? 3 : 2) rescore_
             const unsigned mk = __ballot_sync(0xffffffffu, keep);
             if (count + __popc(mk) > BUF) {  // (only digit rows exceed RBUF)
                 if (lane == 0) P.row_bad[slot] = 1;
-                continue;
+                fits = false;
+                break;
             }
             if (keep) keys[count + __popc(mk & ((1u << lane) - 1u))] = (unsigned long long)(unsigned)cid;
             count += __popc(mk);
