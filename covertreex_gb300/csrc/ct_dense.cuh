@@ -56,8 +56,9 @@ constexpr int kPend = 512;     // pairs of a step that wait for their exact dist
 
 // Tile configurations: QT queries x CT candidates per step, NT threads.  The 256-thread forms run
 // two blocks to an SM, so that one block's epilogue and selection overlap the other's multiply-adds;
-// the 512-thread forms take one SM (rows too wide for half an SM's shared memory).  The 16-row forms
-// serve few queries and the widest rows.
+// the 512-thread forms take one SM (rows too wide for half an SM's shared memory), and so does a
+// launch of the 32-row 256-thread form for rows too wide for the 512-thread one, whose ring and
+// buffers are larger.  The 16-row forms serve few queries and the widest rows.
 enum Cfg { kCfg32 = 0, kCfg16 = 1, kCfg32w = 2, kCfg16w = 3, kNumCfg = 4 };
 template <int C>
 struct CfgOf;
@@ -853,7 +854,7 @@ __device__ __noinline__ void run_tile_v(const Tile& P, u64 nz) {
 
 template <int C>
 __device__ __forceinline__ void run_tile(const Tile& P, u64 nz) {
-    if constexpr (C == kCfg32 || C == kCfg16) {  // (wider rows than m = 256 take the 512-thread forms)
+    if constexpr (C == kCfg32 || C == kCfg16) {  // (wider rows take the general loop or the 512-thread forms)
         if (P.ring.wmax == 64) {
             if (P.m == 64) return run_tile_v<C, 4, 64, 8>(P, nz);
             if (P.m == 128) return run_tile_v<C, 4, 64, 16>(P, nz);

@@ -18,8 +18,8 @@
 // v_x = Li k(Z, x), p_x = var - ||v_x||^2.
 //
 // FP64 on GB300 runs on the CUDA cores only (about two DFMA per clock per SM), so
-// the GEMM is register-tiled 64 x 64 with 4 x 4 outputs per thread and is bound by
-// the DFMA rate; N m^2 FMAs for N rows.
+// the GEMM runs in tiles of 32 x 32 with 2 x 2 outputs per thread (8 or 2 rows for few
+// points) and is bound by the DFMA rate; N m^2 / 2 FMAs for N rows.
 #include <cuda_runtime.h>
 #include <float.h>
 

@@ -162,8 +162,8 @@ class ServingEngine:
         self.rejected: set = set()
         self.evicted: set = set()
         # Stream priorities: dense steps (short, latency-bound) highest, screened requests
-        # two levels below (a screened call runs its exhaustive pass one level above its own
-        # stream), builds lowest, so the block scheduler hands freed SMs to queued step
+        # two levels below (a screened call runs its digit pass and long survivor slots one
+        # level above its own stream), builds lowest, so the block scheduler hands freed SMs to queued step
         # kernels first and to build kernels last (p99 at 500 req/s 6.7-8.3 -> 6.1-6.4 ms
         # against one query priority).
         self.streams = [torch.cuda.Stream(self.device, priority=-3) for _ in range(slots)]
