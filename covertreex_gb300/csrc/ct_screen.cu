@@ -1346,7 +1346,8 @@ __device__ __forceinline__ void pair_bounds_f32(const RescoreParams& P, int q, i
 // a single such slot takes 0.3 to 0.8 ms, which behind the first kernel made calls of fewer than some 20000
 // slots slower than one kernel with full buffers (n = 16384, m = 128, 2000 queries, k = 1: 0.49 ms as one
 // kernel, 0.17 and then 0.42).  Calls of one wave of the full buffers, and m > 512, take one kernel.
-// n = 32768, m = 256: 1.72 ms as one kernel, 1.1 as two.
+// Whole calls, the list behind the rest and beside it: n = 32768, m = 256 5.19 and 4.88 ms; n = 262144, m = 512
+// 107.4 and 106.9 (listed slots 1.7 ms, the rest 10.4; 15.5 as one kernel).
 // Streaming top-k of E through a sorted shared buffer: entries [0, k) hold the current
 // best, new candidates fill the rest, and a full buffer is re-sorted.  Shared memory per
 // warp: BUF keys, then BUF floats (du2, reused for the kept ids).
